@@ -161,6 +161,7 @@ __global__ void __launch_bounds__(256, 2) k_batch_coop(const DeviceScene* __rest
                                                        uint32_t max_depth, BatchBarrier* gb, uint64_t probe_ns) {
     constexpr int WORDS = (int)(sizeof(DeviceScene) / sizeof(uint32_t));
     __shared__ DeviceScene S;
+    __shared__ __align__(8) char s_stack[TRACE_STACK_BYTES<256>];
     const uint32_t nblocks = gridDim.x;
     const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gsize = gridDim.x * blockDim.x;
     const uint64_t limit_ns = probe_ns ? probe_ns : BATCH_BARRIER_NS;
@@ -184,16 +185,16 @@ __global__ void __launch_bounds__(256, 2) k_batch_coop(const DeviceScene* __rest
                 W.hits[idx] = make_float2(s.t_best, __int_as_float(s.best_prim));
             };
             if (d == 0)
-                packet_trace<false>(S, W.rays[0], 3, nrays, &W.ctr[CTR_EFETCH + 0], 0u, nullptr, &W.err[ERR_STACK],
+                packet_trace<false>(S, W.rays[0], 3, nrays, &W.ctr[CTR_EFETCH + 0], &W.err[ERR_STACK],
                                     hit);
             else
-                persistent_trace<false, false, false>(S, W.rays[d & 1], 3, nrays, &W.ctr[CTR_EFETCH + d], 0u, nullptr,
+                persistent_trace<false, false, 256, false>(S, W.rays[d & 1], 3, nrays, &W.ctr[CTR_EFETCH + d], s_stack,
                                                       &W.err[ERR_STACK], W.stats, hit);
             if (!grid_barrier(gb, nblocks, limit_ns)) return;
             shade_stage<false, false, false>(S, F, W, d, C);
             if (!grid_barrier(gb, nblocks, limit_ns)) return;
             const uint32_t nsh = __ldcg(&W.ctr[CTR_SHADOW + d]);
-            persistent_trace<true, false, false>(S, W.shadow, 3, nsh, &W.ctr[CTR_CFETCH + d], 0u, nullptr,
+            persistent_trace<true, false, 256, false>(S, W.shadow, 3, nsh, &W.ctr[CTR_CFETCH + d], s_stack,
                                                  &W.err[ERR_STACK], W.stats, [&](uint32_t idx, const TravState& s) {
                                                      if (s.hit) return;
                                                      const float4* e = W.shadow + 3 * (size_t)idx;
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch_persistent(con
                 TravState ts;
                 int32_t st_ref[CUPBR_STACK_SIZE];
                 float st_t[CUPBR_STACK_SIZE];
-                packet_closest(S, nullptr, 0, xyz(q0), xyz(q1), valid, ts, st_ref, st_t, overflow);
+                packet_closest(S, xyz(q0), xyz(q1), valid, ts, st_ref, st_t, overflow);
                 t = ts.t_best;
                 prim = ts.best_prim;
             }
@@ -289,7 +290,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch_persistent(con
                 for (uint32_t d = 0;; ++d) {
                     if (!PACKET || d > 0) {
                         uint32_t key;
-                        trace_scene_rt(false, false, S, nullptr, 0, xyz(q0), xyz(q1), 0.0f, t, prim, key, overflow,
+                        trace_scene_rt(false, false, S, xyz(q0), xyz(q1), 0.0f, t, prim, key, overflow,
                                        tc);
                     }
                     ShadeOut so;
@@ -298,7 +299,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch_persistent(con
                         float ts;
                         int32_t ps;
                         uint32_t ks;
-                        if (!trace_scene_rt(true, false, S, nullptr, 0, xyz(so.s0), xyz(so.s1), so.s0.w, ts, ps, ks,
+                        if (!trace_scene_rt(true, false, S, xyz(so.s0), xyz(so.s1), so.s0.w, ts, ps, ks,
                                             overflow, tc))
                             rad += xyz(so.s2);
                     }
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch_backward(const
                 float t;
                 int32_t prim;
                 uint32_t key;
-                trace_scene_rt(false, false, S, nullptr, 0, xyz(q0), xyz(q1), 0.0f, t, prim, key, overflow, tc);
+                trace_scene_rt(false, false, S, xyz(q0), xyz(q1), 0.0f, t, prim, key, overflow, tc);
                 ShadeOut so;
                 shade_core<false, false>(S, F, C, d, q0, q1, q2, make_float2(t, __int_as_float(prim)), rad, so);
                 if (so.texel >= 0 && nrec < BATCH_BWD_MAX_DEPTH) {
@@ -413,7 +414,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch_backward(const
                     float ts;
                     int32_t ps;
                     uint32_t ks;
-                    if (!trace_scene_rt(true, false, S, nullptr, 0, xyz(so.s0), xyz(so.s1), so.s0.w, ts, ps, ks,
+                    if (!trace_scene_rt(true, false, S, xyz(so.s0), xyz(so.s1), so.s0.w, ts, ps, ks,
                                         overflow, tc))
                         rad += xyz(so.s2);
                 }

@@ -958,6 +958,36 @@ __global__ void k_write_nodes(const W4* __restrict__ w4, uint32_t n4, const uint
     atomicMax(&st->max_depth, (uint32_t)w.depth + 1);
 }
 
+// Centre and half extent of [lo, hi], rounded outwards: the box they span
+// holds [lo, hi], with 2^-20 of the extent to spare for the traversal's
+// arithmetic on them.  A missing child (inverted bounds) gets half extent
+// -inf, which no slab test accepts; a bound too large to carry its
+// opposite's position gets a box around the origin.
+__device__ __forceinline__ void slab_axis(float lo, float hi, bool empty, float& c, float& h) {
+    if (empty) {
+        c = 0.0f;
+        h = -INFINITY;
+        return;
+    }
+    const float m = fmaxf(fabsf(lo), fabsf(hi));
+    c = m < 1e15f ? 0.5f * lo + 0.5f * hi : 0.0f;
+    h = m < 1e15f ? fmaxf(__fsub_ru(hi, c), __fsub_ru(c, lo)) : m;
+    h = __fmul_ru(h, 1.0f + 1.0f / 1048576.0f);
+}
+
+__global__ void k_slab_nodes(const float4* __restrict__ in, uint32_t n, float4* __restrict__ out) {
+    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= n) return;
+    const float* b = reinterpret_cast<const float*>(in + (size_t)v * BVH_NODE_F4);
+    float* o = reinterpret_cast<float*>(out + (size_t)v * BVH_NODE_F4);
+    for (int k = 0; k < 4; ++k) {
+        const bool empty = __float_as_int(b[24 + k]) == BVH_EMPTY;
+        for (int a = 0; a < 3; ++a) slab_axis(b[8 * a + k], b[8 * a + 4 + k], empty, o[8 * a + k], o[8 * a + 4 + k]);
+        o[24 + k] = b[24 + k];
+        o[28 + k] = 0.0f;
+    }
+}
+
 // Device scratch released on every exit path.
 struct Scratch {
     std::vector<void*> ptrs;
@@ -978,6 +1008,11 @@ struct Scratch {
 inline uint32_t blocks_for(uint64_t n, uint32_t t) { return (uint32_t)std::max<uint64_t>(1, (n + t - 1) / t); }
 
 }  // namespace
+
+cudaError_t launch_slab_nodes(const float4* bounds, uint32_t n, float4* out, cudaStream_t st) {
+    if (n) k_slab_nodes<<<blocks_for(n, 128), 128, 0, st>>>(bounds, n, out);
+    return cudaGetLastError();
+}
 
 bool build_bvh_device(const std::vector<PrimBox>* boxes, int ntypes, const uint32_t* slot_offset,
                       const BvhBuildParams& p, std::vector<uint32_t>* perm, FlatBvh& out, float4** d_nodes,

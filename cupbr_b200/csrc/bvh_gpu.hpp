@@ -29,4 +29,9 @@ bool build_bvh_device(const std::vector<PrimBox>* boxes, int ntypes, const uint3
                       const BvhBuildParams& p, std::vector<uint32_t>* perm, FlatBvh& out, float4** d_nodes,
                       uint32_t* n_nodes, cudaStream_t st, std::string& err);
 
+// The traversal's node array from the builder's (bvh_build.hpp), same order
+// and child references: per axis the four children's centres and half
+// extents instead of their bounds.
+cudaError_t launch_slab_nodes(const float4* bounds, uint32_t n, float4* out, cudaStream_t st);
+
 }  // namespace cupbr_b200

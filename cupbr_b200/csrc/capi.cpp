@@ -137,12 +137,7 @@ struct PTBuffers {
         if ((e = cudaMemset(p, 0, sizeof(uint32_t) * ERR_TOTAL)) != cudaSuccess) return e;
         if ((e = alloc(&p, sizeof(uint64_t) * STAT_TOTAL)) != cudaSuccess) return e;
         ws.stats = (uint64_t*)p;
-        // no BVH nodes staged in shared memory: with the top 128 nodes
-        // staged (16 KB per block) the 1080p heightfield frame measured 3 %
-        // slower than with none (the L1 left to the traversal stacks and
-        // node loads serves the top of the tree as well)
-        ws.smem_nodes = 0;
-        ws.trace_blocks_per_sm = pt_occupancy_blocks((int)(ws.smem_nodes * BVH_NODE_BYTES));
+        ws.trace_blocks_per_sm = pt_occupancy_blocks();
         capacity = n;
         return cudaSuccess;
     }
@@ -622,7 +617,7 @@ int cupbr_scene_get_bvh(cupbr_scene_t s, float* out, uint32_t cap, uint32_t* n_n
     *n_nodes = s->g.dev.n_nodes;
     if (!out) return CUPBR_OK;
     if (cap < s->g.dev.n_nodes) return fail(CUPBR_ERR_ARG, "capacity too small");
-    CUPBR_CHECK_CUDA(cudaMemcpy(out, s->g.dev.nodes, (size_t)s->g.dev.n_nodes * BVH_NODE_BYTES, cudaMemcpyDeviceToHost));
+    CUPBR_CHECK_CUDA(cudaMemcpy(out, s->g.bounds, (size_t)s->g.dev.n_nodes * BVH_NODE_BYTES, cudaMemcpyDeviceToHost));
     return CUPBR_OK;
 }
 int cupbr_scene_get_key_slots(cupbr_scene_t s, uint32_t* out, uint32_t cap, uint32_t* n_keys) {
@@ -1785,7 +1780,7 @@ struct cupbr_batch_s {
         for (const BatchWave& w : waves) need = std::max(need, w.n_paths);
         cudaError_t e = pt.ensure(need);
         if (e != cudaSuccess) return e;
-        const int full = pt_occupancy_blocks((int)(pt.ws.smem_nodes * BVH_NODE_BYTES));
+        const int full = pt_occupancy_blocks();
         pt.ws.trace_blocks_per_sm = std::max(1, (int)(full * trace_share + 0.5f));
         if ((e = dev_alloc(&dsegs, sizeof(BatchSegment) * std::max<size_t>(1, segs.size()))) != cudaSuccess) return e;
         if (!segs.empty() &&

@@ -61,6 +61,26 @@ struct HostArray {
     bool empty() const { return n == 0; }
 };
 
+// The traversal's form of the committed tree's nodes (dev.nodes).
+bool make_slab_nodes(GpuScene& g, std::string& err) {
+    g.dev.nodes = nullptr;
+    if (g.dev.n_nodes == 0) return true;
+    const size_t bytes = (size_t)g.dev.n_nodes * BVH_NODE_BYTES;
+    void* p = nullptr;
+    cudaError_t e = dev_alloc(&p, bytes);
+    if (e == cudaSuccess) {
+        g.buffers.push_back(p);
+        g.device_bytes += bytes;
+        e = launch_slab_nodes(g.bounds, g.dev.n_nodes, static_cast<float4*>(p), 0);
+    }
+    if (e != cudaSuccess) {
+        err = std::string("traversal nodes: ") + cudaGetErrorString(e);
+        return false;
+    }
+    g.dev.nodes = static_cast<const float4*>(p);
+    return true;
+}
+
 template <typename Cont, typename T>
 bool upload(GpuScene& g, const Cont& v, const T*& out, std::string& err) {
     if (v.empty()) { out = nullptr; return true; }
@@ -379,15 +399,16 @@ bool commit_scene(GpuScene& g, const BvhBuildParams& params, std::string& err) {
     DeviceScene& D = g.dev;
     const F4* p;
     if (dev_nodes) {
-        D.nodes = dev_nodes;
+        g.bounds = dev_nodes;
         D.n_nodes = dev_n_nodes;
     } else {
         std::vector<F4> nodes(g.bvh.nodes.size() / 4);
         std::memcpy(nodes.data(), g.bvh.nodes.data(), g.bvh.nodes.size() * sizeof(float));
         if (!upload(g, nodes, p, err)) return false;
-        D.nodes = reinterpret_cast<const float4*>(p);
+        g.bounds = reinterpret_cast<const float4*>(p);
         D.n_nodes = (uint32_t)(nodes.size() / BVH_NODE_F4);  // nodes, not float4s
     }
+    if (!make_slab_nodes(g, err)) return false;
     if (!upload(g, tris, p, err)) return false;
     D.tris = reinterpret_cast<const float4*>(p);
     if (!upload(g, trin, p, err)) return false;

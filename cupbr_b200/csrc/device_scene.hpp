@@ -19,6 +19,7 @@ struct GpuScene {
     BvhBuildParams params;           // BVH parameters of the last commit
     uint64_t generation = 0;         // incremented by every commit (device buffers replaced)
     DeviceScene dev{};
+    const float4* bounds = nullptr;  // dev.n_nodes builder nodes (child bounds, bvh_build.hpp)
     std::vector<void*> buffers;
     FlatBvh bvh;
     uint64_t device_bytes = 0;

@@ -657,13 +657,12 @@ __global__ void __launch_bounds__(PT_TRACE_THREADS) k_medium_connect(DeviceScene
                                                                      const float* __restrict__ grad_img,
                                                                      float* g_grid, float* g_params, uint32_t np_smem,
                                                                      uint32_t* err) {
-    extern __shared__ float4 s_dyn[];
-    const uint32_t nsm = min(S.n_nodes, W.smem_nodes);
-    float* s_params = reinterpret_cast<float*>(s_dyn + BVH_NODE_F4 * nsm);
+    extern __shared__ float s_params[];
+    __shared__ __align__(8) char s_stack[LaneStack<true, PT_TRACE_THREADS>::NEAR];
     float* gp = params_begin(s_params, np_smem, g_params);
     bool ovf = false;
-    persistent_trace<true, false>(
-        S, W.shadow, 3, W.ctr[CTR_SHADOW + depth], &W.ctr[CTR_CFETCH + depth], W.smem_nodes, s_dyn,
+    persistent_trace<true, false, PT_TRACE_THREADS>(
+        S, W.shadow, 3, W.ctr[CTR_SHADOW + depth], &W.ctr[CTR_CFETCH + depth], s_stack,
         &W.err[ERR_STACK], W.stats, [&](uint32_t idx, const TravState& s) {
             if (s.hit) return;
             const float4* e = W.shadow + 3 * (size_t)idx;
@@ -737,7 +736,7 @@ cudaError_t wavefront(const DeviceScene& S, const MediumGrid& G, const MediumPar
                       int num_sms, cudaStream_t st, Mark mark) {
     const uint32_t np = medium_param_count(S.n_objects, S.n_lights);
     const uint32_t np_smem = MODE == ADJOINT && np <= MEDIUM_SMEM_PARAMS ? np : 0;
-    const int connect_smem = (int)(std::min(S.n_nodes, W.pt.smem_nodes) * BVH_NODE_BYTES + np_smem * sizeof(float));
+    const int connect_smem = (int)(np_smem * sizeof(float));
     unsigned long long* stats = MODE == RENDER ? W.stats : nullptr;
     cudaError_t e = cudaMemsetAsync(W.pt.ctr, 0, sizeof(uint32_t) * CTR_TOTAL, st);
     if (e != cudaSuccess) return e;

@@ -68,7 +68,7 @@ __device__ __noinline__ RtOut trace_call(bool any, bool count, const DeviceScene
     TraceCounters c;
     uint32_t key;
     r.ovf = false;
-    r.hit = trace_scene_rt(any, count, S, nullptr, 0, o, d, t_limit, r.t, r.prim, key, r.ovf, c);
+    r.hit = trace_scene_rt(any, count, S, o, d, t_limit, r.t, r.prim, key, r.ovf, c);
     r.nodes = c.nodes;
     r.tris = c.tris;
     return r;

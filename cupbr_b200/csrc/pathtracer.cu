@@ -23,8 +23,7 @@
 //
 // Queue slots are claimed with warp-aggregated atomics (one atomicAdd per
 // warp, ballot + popc for the lane offsets); the traversal kernels are
-// persistent and fetch 32 rays per warp from a global counter, with the top
-// of the BVH staged in shared memory.
+// persistent (persistent_trace).
 #include "pathtracer.hpp"
 
 #include "cache.hpp"
@@ -42,8 +41,8 @@ __global__ void k_camera(PTFrame F, Workspace W) {
     const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (slot == 0) W.ctr[CTR_RAYS + 0] = F.n_paths;
     if (slot >= F.n_paths) return;
-    const uint32_t fr = slot / F.pixels;
-    const uint32_t tid = slot_pixel(slot - fr * F.pixels, F.width, F.height);
+    uint32_t fr, tid;
+    slot_path(slot, F.width, F.height, F.frames, fr, tid);
     const uint32_t p = fr * F.pixels + tid;  // path
     // TracingDetail.h:15-30 (index2pixel: KernelHelperDetail.h:13-20)
     uint32_t seed = tea4(tid, F.frame_index + fr);
@@ -65,12 +64,12 @@ __global__ void k_camera(PTFrame F, Workspace W) {
 // Closest hit of ray queue[depth] into the hit buffer (persistent, dynamic
 // fetch; see persistent_trace).
 template <bool COUNT>
-__global__ void __launch_bounds__(PT_TRACE_THREADS) k_extend(DeviceScene S, Workspace W, uint32_t depth,
+__global__ void __launch_bounds__(PT_TRACE_THREADS, 8) k_extend(DeviceScene S, Workspace W, uint32_t depth,
                                                               uint32_t min_count) {
     if (W.ctr[CTR_RAYS + depth] < min_count) return;  // cached frames: left to k_tail
-    extern __shared__ float4 s_nodes[];
-    persistent_trace<false, COUNT>(S, W.rays[depth & 1], 3, W.ctr[CTR_RAYS + depth], &W.ctr[CTR_EFETCH + depth],
-                                   W.smem_nodes, s_nodes, &W.err[ERR_STACK], W.stats + STAT_EXT_NODES,
+    __shared__ __align__(8) char s_stack[TRACE_STACK_BYTES<PT_TRACE_THREADS>];
+    persistent_trace<false, COUNT, PT_TRACE_THREADS>(S, W.rays[depth & 1], 3, W.ctr[CTR_RAYS + depth], &W.ctr[CTR_EFETCH + depth],
+                                   s_stack, &W.err[ERR_STACK], W.stats + STAT_EXT_NODES,
                                    [&](uint32_t idx, const TravState& s) {
                                        W.hits[idx] = make_float2(s.t_best, __int_as_float(s.best_prim));
                                    });
@@ -80,23 +79,24 @@ __global__ void __launch_bounds__(PT_TRACE_THREADS) k_extend(DeviceScene S, Work
 // fills 32 consecutive slots from one 8x4 pixel tile (packet_trace).
 __global__ void __launch_bounds__(PT_TRACE_THREADS) k_extend_camera(DeviceScene S, Workspace W, uint32_t min_count) {
     if (W.ctr[CTR_RAYS + 0] < min_count) return;  // cached frames: left to k_tail
-    extern __shared__ float4 s_nodes[];
-    packet_trace(S, W.rays[0], 3, W.ctr[CTR_RAYS + 0], &W.ctr[CTR_EFETCH + 0], W.smem_nodes, s_nodes,
-                 &W.err[ERR_STACK], [&](uint32_t idx, const TravState& s) {
+    packet_trace(S, W.rays[0], 3, W.ctr[CTR_RAYS + 0], &W.ctr[CTR_EFETCH + 0], &W.err[ERR_STACK],
+                 [&](uint32_t idx, const TravState& s) {
                      W.hits[idx] = make_float2(s.t_best, __int_as_float(s.best_prim));
                  });
 }
 
 // Shadow queue of depth: visible contributions are added to the path
 // radiance (TracingDetail.h:181-182 visible -> PathTracer.cu:66-72).
-// Held at 8 blocks per SM (64 registers) like the closest-hit kernels, which
-// set the traversal grid: unconstrained it takes 72 registers, 7 blocks fit
-// and the eighth of the grid starts late.
+// Both traversal kernels are held at 8 blocks per SM (64 registers): at 9 or
+// 10 the spills cost more than the warps give (1080p terrain 45.4 -> 48.3 /
+// 55.3 ms).  Adding the contribution by a vector reduction
+// instead of a load and a store keeps the shadow queue's counter waiting
+// behind it (scene of 20 primitives: stage 1.17 -> 1.40 ms).
 template <bool COUNT>
 __global__ void __launch_bounds__(PT_TRACE_THREADS, 8) k_connect(DeviceScene S, Workspace W, uint32_t depth) {
-    extern __shared__ float4 s_nodes[];
-    persistent_trace<true, COUNT>(S, W.shadow, 3, W.ctr[CTR_SHADOW + depth], &W.ctr[CTR_CFETCH + depth], W.smem_nodes,
-                                  s_nodes, &W.err[ERR_STACK], W.stats + STAT_SH_NODES,
+    __shared__ __align__(8) char s_stack[LaneStack<true, PT_TRACE_THREADS>::NEAR];
+    persistent_trace<true, COUNT, PT_TRACE_THREADS>(S, W.shadow, 3, W.ctr[CTR_SHADOW + depth], &W.ctr[CTR_CFETCH + depth], s_stack,
+                                  &W.err[ERR_STACK], W.stats + STAT_SH_NODES,
                                   [&](uint32_t idx, const TravState& s) {
                                       if (s.hit) return;
                                       const float4* e = W.shadow + 3 * (size_t)idx;
@@ -134,14 +134,14 @@ __global__ void __launch_bounds__(128) k_tail(DeviceScene S, PTFrame F, Workspac
             float t;
             int32_t prim;
             uint32_t key;
-            trace_scene_rt(false, false, S, nullptr, 0, xyz(q0), xyz(q1), 0.0f, t, prim, key, overflow, tc);
+            trace_scene_rt(false, false, S, xyz(q0), xyz(q1), 0.0f, t, prim, key, overflow, tc);
             ShadeOut so;
             shade_one<CACHE, PHYS>(S, F, W, C, d, q0, q1, q2, make_float2(t, __int_as_float(prim)), so);
             if (so.sh) {
                 float ts;
                 int32_t ps;
                 uint32_t ks;
-                const bool hit = trace_scene_rt(true, false, S, nullptr, 0, xyz(so.s0), xyz(so.s1), so.s0.w, ts, ps,
+                const bool hit = trace_scene_rt(true, false, S, xyz(so.s0), xyz(so.s1), so.s0.w, ts, ps,
                                                 ks, overflow, tc);
                 if (!hit) {
                     const uint32_t pid = __float_as_uint(so.s1.w);
@@ -199,10 +199,10 @@ __global__ void k_trace_rays(DeviceScene S, uint32_t n, const float* __restrict_
     bool overflow = false;
     TraceCounters tc;
     if (dist) {
-        bool occ = trace_scene<true, false>(S, nullptr, 0, org, dir, dist[i], t, prim, key, overflow, tc);
+        bool occ = trace_scene<true, false>(S, org, dir, dist[i], t, prim, key, overflow, tc);
         vis_out[i] = occ ? 0 : 1;
     } else {
-        trace_scene<false, false>(S, nullptr, 0, org, dir, 0.0f, t, prim, key, overflow, tc);
+        trace_scene<false, false>(S, org, dir, 0.0f, t, prim, key, overflow, tc);
         t_out[i] = t;
         prim_out[i] = prim;
         key_out[i] = key;
@@ -224,16 +224,14 @@ cudaError_t launch_trace_rays(const DeviceScene& S, uint32_t n, const float* o, 
 
 cudaError_t pt_launch_extend(const DeviceScene& S, const Workspace& W, uint32_t depth, int num_sms, cudaStream_t st,
                              uint32_t min_count, bool count) {
-    const int smem = (int)(std::min(S.n_nodes, W.smem_nodes) * BVH_NODE_BYTES);
-    if (count) k_extend<true><<<num_sms * W.trace_blocks_per_sm, PT_TRACE_THREADS, smem, st>>>(S, W, depth, min_count);
-    else k_extend<false><<<num_sms * W.trace_blocks_per_sm, PT_TRACE_THREADS, smem, st>>>(S, W, depth, min_count);
+    if (count) k_extend<true><<<num_sms * W.trace_blocks_per_sm, PT_TRACE_THREADS, 0, st>>>(S, W, depth, min_count);
+    else k_extend<false><<<num_sms * W.trace_blocks_per_sm, PT_TRACE_THREADS, 0, st>>>(S, W, depth, min_count);
     return cudaGetLastError();
 }
 
 cudaError_t pt_launch_extend_camera(const DeviceScene& S, const Workspace& W, int num_sms, cudaStream_t st,
                                     uint32_t min_count) {
-    const int smem = (int)(std::min(S.n_nodes, W.smem_nodes) * BVH_NODE_BYTES);
-    k_extend_camera<<<num_sms * W.trace_blocks_per_sm, PT_TRACE_THREADS, smem, st>>>(S, W, min_count);
+    k_extend_camera<<<num_sms * W.trace_blocks_per_sm, PT_TRACE_THREADS, 0, st>>>(S, W, min_count);
     return cudaGetLastError();
 }
 
@@ -247,9 +245,8 @@ cudaError_t pt_launch_tail(const DeviceScene& S, const PTFrame& F, const Workspa
 
 cudaError_t pt_launch_connect(const DeviceScene& S, const Workspace& W, uint32_t depth, int num_sms, cudaStream_t st,
                               bool count) {
-    const int smem = (int)(std::min(S.n_nodes, W.smem_nodes) * BVH_NODE_BYTES);
-    if (count) k_connect<true><<<num_sms * W.trace_blocks_per_sm, PT_TRACE_THREADS, smem, st>>>(S, W, depth);
-    else k_connect<false><<<num_sms * W.trace_blocks_per_sm, PT_TRACE_THREADS, smem, st>>>(S, W, depth);
+    if (count) k_connect<true><<<num_sms * W.trace_blocks_per_sm, PT_TRACE_THREADS, 0, st>>>(S, W, depth);
+    else k_connect<false><<<num_sms * W.trace_blocks_per_sm, PT_TRACE_THREADS, 0, st>>>(S, W, depth);
     return cudaGetLastError();
 }
 
@@ -276,9 +273,9 @@ cudaError_t pt_launch_accumulate(const PTFrame& F, const Workspace& W, float* im
     return cudaGetLastError();
 }
 
-int pt_occupancy_blocks(int smem_bytes) {
+int pt_occupancy_blocks() {
     int b = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_extend<false>, PT_TRACE_THREADS, smem_bytes);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_extend<false>, PT_TRACE_THREADS, 0);
     return b > 0 ? b : 1;
 }
 
@@ -293,7 +290,6 @@ cudaError_t pt_render_frame(const DeviceScene& S, const PTFrame& F, const Worksp
     mark();
     k_camera<<<nb, 256, 0, st>>>(F, W);
     mark();
-    const int smem = (int)(std::min(S.n_nodes, W.smem_nodes) * BVH_NODE_BYTES);
     const int trace_blocks = num_sms * W.trace_blocks_per_sm;
     const int shade_blocks = num_sms * 8;
     // instrumented frames count every ray's traversal: no tail there
@@ -305,15 +301,15 @@ cudaError_t pt_render_frame(const DeviceScene& S, const PTFrame& F, const Worksp
             if (F.estimator) k_tail<false, true><<<tail_blocks, 128, 0, st>>>(S, F, W, d, T);
             else k_tail<false, false><<<tail_blocks, 128, 0, st>>>(S, F, W, d, T);
         }
-        if (count_stats) k_extend<true><<<trace_blocks, PT_TRACE_THREADS, smem, st>>>(S, W, d, 0u);
-        else if (d == 0) k_extend_camera<<<trace_blocks, PT_TRACE_THREADS, smem, st>>>(S, W, T.tail_threshold);
-        else k_extend<false><<<trace_blocks, PT_TRACE_THREADS, smem, st>>>(S, W, d, T.tail_threshold);
+        if (count_stats) k_extend<true><<<trace_blocks, PT_TRACE_THREADS, 0, st>>>(S, W, d, 0u);
+        else if (d == 0) k_extend_camera<<<trace_blocks, PT_TRACE_THREADS, 0, st>>>(S, W, T.tail_threshold);
+        else k_extend<false><<<trace_blocks, PT_TRACE_THREADS, 0, st>>>(S, W, d, T.tail_threshold);
         mark();
         if (F.estimator) k_shade<false, true><<<shade_blocks, 256, 0, st>>>(S, F, W, d, T);
         else k_shade<false, false><<<shade_blocks, 256, 0, st>>>(S, F, W, d, T);
         mark();
-        if (count_stats) k_connect<true><<<trace_blocks, PT_TRACE_THREADS, smem, st>>>(S, W, d);
-        else k_connect<false><<<trace_blocks, PT_TRACE_THREADS, smem, st>>>(S, W, d);
+        if (count_stats) k_connect<true><<<trace_blocks, PT_TRACE_THREADS, 0, st>>>(S, W, d);
+        else k_connect<false><<<trace_blocks, PT_TRACE_THREADS, 0, st>>>(S, W, d);
         mark();
     }
     if (img) k_accumulate<<<(F.pixels + 255) / 256, 256, 0, st>>>(F, W, img);

@@ -49,11 +49,10 @@ struct Workspace {
     uint32_t* ctr;         // CTR_TOTAL counters
     uint32_t* err;         // ERR_TOTAL error counters (never reset by a frame)
     uint64_t* stats;       // STAT_TOTAL traversal counters (instrumented frames only)
-    uint32_t smem_nodes;   // BVH nodes staged in shared memory per block
     int trace_blocks_per_sm;
 };
 
-int pt_occupancy_blocks(int smem_bytes);
+int pt_occupancy_blocks();
 // The path tracer's persistent traversal stages on their own: closest hits of
 // ray queue[depth] into W.hits, and the shadow queue of depth (3 float4 per
 // entry: (origin, distance), (direction, path), (contribution, -)) with the

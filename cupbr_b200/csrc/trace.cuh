@@ -11,7 +11,7 @@
 // depth-first order, then triangle index, MeshDetail.h:28-35).
 //
 // The SAH BVH itself is traversed with conservative FMA slab tests against
-// boxes that the builder inflated, a per-thread short stack of (node, t_near)
+// boxes that the builder inflated, a per-thread short stack of (t_near, node)
 // entries and near-child-first ordering.
 #pragma once
 
@@ -204,75 +204,133 @@ __device__ __forceinline__ float safe_inv(float v) {
     return 1.0f / (fabsf(v) > 1e-20f ? v : copysignf(1e-20f, v));
 }
 
-// Node fetch (the 7 used float4s of a 4-wide node, bvh_build.hpp): the
-// first `nsm` nodes are staged in shared memory.
-__device__ __forceinline__ void fetch_node(const DeviceScene& S, const float4* __restrict__ snodes, uint32_t nsm,
-                                           int32_t idx, float4* nb) {
-    if ((uint32_t)idx < nsm) {
-        const float4* p = snodes + BVH_NODE_F4 * idx;
-#pragma unroll
-        for (int k = 0; k < 7; ++k) nb[k] = p[k];
-    } else {
-        const float4* p = S.nodes + BVH_NODE_F4 * (size_t)idx;
-#pragma unroll
-        for (int k = 0; k < 7; ++k) nb[k] = __ldg(p + k);
-    }
+// The two float4s of one 32-byte row of a node (lo and hi bounds of one axis)
+// in one 256-bit load (128-byte aligned nodes).
+__device__ __forceinline__ void ld_row(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(__cvta_generic_to_global(p)));
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
 }
 
-// Slab tests of a 4-wide node's children (t in [0, lim], FMA form on the
-// conservatively inflated boxes).  Returns false when no child is hit;
-// otherwise `first` is the nearest child hit and the others are pushed
-// far-to-near (the nearest of them on top), each with its entry distance.
-// KEEP_T = false (occlusion rays, whose limit never shrinks, so every entry
-// pushed stays within it): the entry distances are not stored and the
-// children are visited in node order.
-template <bool KEEP_T = true>
-__device__ __forceinline__ bool visit4(const float4* nb, f3 idir, f3 ood, float lim, int32_t& first, int32_t* st_ref,
-                                       float* st_t, int& sp, bool& overflow) {
-    const float INF = __int_as_float(0x7f800000);
-    const float lx[4] = {nb[0].x, nb[0].y, nb[0].z, nb[0].w}, hx[4] = {nb[1].x, nb[1].y, nb[1].z, nb[1].w};
-    const float ly[4] = {nb[2].x, nb[2].y, nb[2].z, nb[2].w}, hy[4] = {nb[3].x, nb[3].y, nb[3].z, nb[3].w};
-    const float lz[4] = {nb[4].x, nb[4].y, nb[4].z, nb[4].w}, hz[4] = {nb[5].x, nb[5].y, nb[5].z, nb[5].w};
-    int32_t r0 = __float_as_int(nb[6].x), r1 = __float_as_int(nb[6].y), r2 = __float_as_int(nb[6].z),
-            r3 = __float_as_int(nb[6].w);
-    float key[4];
+// A ray as the slab tests read it: 1 / d, o / d and |1 / d|.
+struct SlabRay {
+    f3 i, o, a;
+};
+__device__ __forceinline__ SlabRay slab_ray(f3 o, f3 d) {
+    SlabRay r;
+    r.i = mk(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
+    r.o = mk(o.x * r.i.x, o.y * r.i.y, o.z * r.i.z);
+    r.a = mk(fabsf(r.i.x), fabsf(r.i.y), fabsf(r.i.z));
+    return r;
+}
+
+// Slab tests of a 4-wide node's children (t in [0, lim]): entry distances and
+// which are hit.  The boxes come as centres and half extents, so entry and
+// exit follow from the distance to the centre plane by one fused multiply-add
+// each: 12 more of those per node than with the two planes of each slab, and
+// 24 fewer minima and maxima, which run at half their rate and kept the
+// integer / compare pipe 63 % busy (43 % now).  A node is read with three
+// 256-bit loads and one of 128.  Packing two children into one
+// fma.rn.f32x2 halves the multiply-adds again, but its operand pairs did not
+// fit the register budget (1080p terrain 45.4 -> 47.8 ms).
+struct Slab4 {
+    float tn[4];
+    bool hit[4];
+    int32_t ref[4];
+};
+__device__ __forceinline__ Slab4 slab4(const float4* __restrict__ node, const SlabRay& r, float lim) {
+    float4 cx, hx, cy, hy, cz, hz;
+    ld_row(node, cx, hx);
+    ld_row(node + 2, cy, hy);
+    ld_row(node + 4, cz, hz);
+    const int4 rf = __ldg(reinterpret_cast<const int4*>(node + 6));
+    const float x[4] = {cx.x, cx.y, cx.z, cx.w}, ex[4] = {hx.x, hx.y, hx.z, hx.w};
+    const float y[4] = {cy.x, cy.y, cy.z, cy.w}, ey[4] = {hy.x, hy.y, hy.z, hy.w};
+    const float z[4] = {cz.x, cz.y, cz.z, cz.w}, ez[4] = {hz.x, hz.y, hz.z, hz.w};
+    Slab4 s;
+    s.ref[0] = rf.x; s.ref[1] = rf.y; s.ref[2] = rf.z; s.ref[3] = rf.w;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const float x0 = __fmaf_rn(lx[k], idir.x, -ood.x), x1 = __fmaf_rn(hx[k], idir.x, -ood.x);
-        const float y0 = __fmaf_rn(ly[k], idir.y, -ood.y), y1 = __fmaf_rn(hy[k], idir.y, -ood.y);
-        const float z0 = __fmaf_rn(lz[k], idir.z, -ood.z), z1 = __fmaf_rn(hz[k], idir.z, -ood.z);
-        const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), 0.0f));
-        const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), lim));
-        key[k] = tn <= tf ? tn : INF;
+        const float mx = __fmaf_rn(x[k], r.i.x, -r.o.x), my = __fmaf_rn(y[k], r.i.y, -r.o.y),
+                    mz = __fmaf_rn(z[k], r.i.z, -r.o.z);
+        s.tn[k] = fmaxf(max3(__fmaf_rn(-ex[k], r.a.x, mx), __fmaf_rn(-ey[k], r.a.y, my), __fmaf_rn(-ez[k], r.a.z, mz)),
+                        0.0f);
+        const float tf = fminf(min3(__fmaf_rn(ex[k], r.a.x, mx), __fmaf_rn(ey[k], r.a.y, my),
+                                    __fmaf_rn(ez[k], r.a.z, mz)), lim);
+        s.hit[k] = s.tn[k] <= tf;
     }
-    // a missing child has an inverted box, which a min/max slab test could
-    // still accept, so it is excluded by its reference
-    if (r0 == BVH_EMPTY) key[0] = INF;
-    if (r1 == BVH_EMPTY) key[1] = INF;
-    if (r2 == BVH_EMPTY) key[2] = INF;
-    if (r3 == BVH_EMPTY) key[3] = INF;
-    if (!KEEP_T) {
-        // occlusion rays: any counted hit ends the ray, so the children are
-        // not ordered by entry distance (measured faster than near-first:
-        // k_connect 0.726 -> 0.700 ms per 1080p frame of the heightfield);
-        // the first accepted child is entered, the others pushed
-        const int lowest = key[0] < INF ? 0 : key[1] < INF ? 1 : key[2] < INF ? 2 : key[3] < INF ? 3 : -1;
+    return s;
+}
+
+// Traversal stacks.  An entry is (entry distance's bits, child reference):
+// entry distances are >= 0, so their bits order as integers; occlusion rays
+// keep the reference only.
+constexpr int32_t KEY_MISS = 0x7fffffff;
+// An entry can still hold a counted hit while its key is at most this.
+__device__ __forceinline__ int32_t key_limit(float t_best) { return __float_as_int(t_best) & 0x7fffffff; }
+
+struct LocalStack {
+    int2 e[CUPBR_STACK_SIZE];
+    int sp;
+    __device__ __forceinline__ void clear() { sp = 0; }
+    __device__ __forceinline__ bool empty() const { return sp == 0; }
+    static constexpr int ROW = 1;
+    __device__ __forceinline__ bool near3() const { return sp <= CUPBR_STACK_SIZE - 3; }
+    __device__ __forceinline__ void put(int at, int32_t key, int32_t ref) { e[at] = make_int2(key, ref); }
+    __device__ __forceinline__ void push(int32_t key, int32_t ref, bool& overflow) {
+        if (sp < CUPBR_STACK_SIZE) e[sp++] = make_int2(key, ref);
+        else overflow = true;
+    }
+    __device__ __forceinline__ int2 pop() { return e[--sp]; }
+};
+
+// Enters a node: `first` is the child to visit next (nearest first; any order
+// for occlusion rays, where any counted hit ends the ray) and the other
+// children hit are pushed far-to-near.  False when no child is hit.
+template <bool ANY, typename Stack>
+__device__ __forceinline__ bool visit4(const float4* __restrict__ node, const SlabRay& r, float lim, int32_t& first,
+                                       Stack& st, bool& overflow) {
+    const Slab4 s = slab4(node, r, lim);
+    if (ANY) {
+        const int lowest = s.hit[0] ? 0 : s.hit[1] ? 1 : s.hit[2] ? 2 : s.hit[3] ? 3 : -1;
         if (lowest < 0) return false;
-        const int32_t rr[4] = {r0, r1, r2, r3};
-        first = rr[lowest];
+        first = s.hit[0] ? s.ref[0] : s.hit[1] ? s.ref[1] : s.hit[2] ? s.ref[2] : s.ref[3];
+        if (st.near3()) {
 #pragma unroll
-        for (int k = 3; k >= 0; --k) {
-            if (k == lowest || !(key[k] < INF)) continue;
-            if (sp < CUPBR_STACK_SIZE) st_ref[sp++] = rr[k];
-            else overflow = true;
+            for (int k = 3; k >= 1; --k)
+                if (s.hit[k] && k != lowest) {
+                    st.put(st.sp, 0, s.ref[k]);
+                    st.sp += Stack::ROW;
+                }
+        } else {
+            for (int k = 3; k >= 1; --k)
+                if (s.hit[k] && k != lowest) st.push(0, s.ref[k], overflow);
         }
         return true;
     }
-    float k0 = key[0], k1 = key[1], k2 = key[2], k3 = key[3];
-#define CUPBR_CSWAP(ka, ra, kb, rb)              \
-    if (kb < ka) {                               \
-        const float tk = ka; ka = kb; kb = tk;   \
-        const int32_t tr = ra; ra = rb; rb = tr; \
+    int32_t k[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) k[c] = s.hit[c] ? __float_as_int(s.tn[c]) : KEY_MISS;
+    int32_t k0 = k[0], k1 = k[1], k2 = k[2], k3 = k[3];
+    int32_t r0 = s.ref[0], r1 = s.ref[1], r2 = s.ref[2], r3 = s.ref[3];
+#define CUPBR_CSWAP(ka, ra, kb, rb)                        \
+    {                                                      \
+        const bool w_ = kb < ka;                           \
+        const int32_t lo_ = min(ka, kb), rl_ = w_ ? rb : ra; \
+        kb = max(ka, kb);                                  \
+        rb = w_ ? ra : rb;                                 \
+        ka = lo_;                                          \
+        ra = rl_;                                          \
     }
     CUPBR_CSWAP(k0, r0, k1, r1)
     CUPBR_CSWAP(k2, r2, k3, r3)
@@ -280,20 +338,17 @@ __device__ __forceinline__ bool visit4(const float4* nb, f3 idir, f3 ood, float 
     CUPBR_CSWAP(k1, r1, k3, r3)
     CUPBR_CSWAP(k1, r1, k2, r2)
 #undef CUPBR_CSWAP
-    if (!(k0 < INF)) return false;
+    if (k0 == KEY_MISS) return false;
     first = r0;
-    const float ks[3] = {k3, k2, k1};
-    const int32_t rs[3] = {r3, r2, r1};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        if (!(ks[k] < INF)) continue;
-        if (sp < CUPBR_STACK_SIZE) {
-            st_ref[sp] = rs[k];
-            if (KEEP_T) st_t[sp] = ks[k];
-            ++sp;
-        } else {
-            overflow = true;
-        }
+    if (st.near3()) {
+        st.sp += (k3 != KEY_MISS ? 3 : k2 != KEY_MISS ? 2 : k1 != KEY_MISS ? 1 : 0) * Stack::ROW;
+        if (k1 != KEY_MISS) st.put(st.sp - Stack::ROW, k1, r1);
+        if (k2 != KEY_MISS) st.put(st.sp - 2 * Stack::ROW, k2, r2);
+        if (k3 != KEY_MISS) st.put(st.sp - 3 * Stack::ROW, k3, r3);
+    } else {
+        if (k3 != KEY_MISS) st.push(k3, r3, overflow);
+        if (k2 != KEY_MISS) st.push(k2, r2, overflow);
+        if (k1 != KEY_MISS) st.push(k1, r1, overflow);
     }
     return true;
 }
@@ -307,10 +362,9 @@ __device__ __forceinline__ bool visit4(const float4* nb, f3 idir, f3 ood, float 
 // trace_scene_rt takes ANY / COUNT at run time, for kernels that trace
 // closest-hit and shadow rays from one call site (one copy of the loop in
 // the instruction cache); with constant flags it folds to trace_scene.
-__device__ __forceinline__ bool trace_scene_rt(bool ANY, bool COUNT, const DeviceScene& S,
-                                               const float4* __restrict__ snodes, uint32_t nsm, f3 o, f3 d,
-                                               float t_limit, float& t_best, int32_t& best_prim, uint32_t& best_key,
-                                               bool& overflow, TraceCounters& ctr) {
+__device__ __forceinline__ bool trace_scene_rt(bool ANY, bool COUNT, const DeviceScene& S, f3 o, f3 d, float t_limit,
+                                               float& t_best, int32_t& best_prim, uint32_t& best_key, bool& overflow,
+                                               TraceCounters& ctr) {
     RefBoxCache cache;
     t_best = ANY ? t_limit : __int_as_float(0x7f800000);
     best_prim = HIT_NONE;
@@ -331,12 +385,9 @@ __device__ __forceinline__ bool trace_scene_rt(bool ANY, bool COUNT, const Devic
     }
     if (S.n_nodes == 0) return ANY ? false : best_prim != HIT_NONE;
 
-    const f3 idir = mk(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
-    const f3 ood = mk(o.x * idir.x, o.y * idir.y, o.z * idir.z);
-
-    int32_t st_ref[CUPBR_STACK_SIZE];
-    float st_t[CUPBR_STACK_SIZE];
-    int sp = 0;
+    const SlabRay sr = slab_ray(o, d);
+    LocalStack st;
+    st.clear();
     int32_t cur = 0;
     // A well-formed tree visits every node at most once per ray; the bound
     // turns a malformed node array into a reported error instead of a hang.
@@ -352,11 +403,9 @@ __device__ __forceinline__ bool trace_scene_rt(bool ANY, bool COUNT, const Devic
                 overflow = true;
                 return ANY ? false : best_prim != HIT_NONE;
             }
-            float4 nb[7];
-            fetch_node(S, snodes, nsm, cur, nb);
             if (COUNT) ctr.nodes++;
             int32_t first;
-            if (visit4(nb, idir, ood, t_best, first, st_ref, st_t, sp, overflow)) {
+            if (visit4<false>(S.nodes + BVH_NODE_F4 * (size_t)cur, sr, t_best, first, st, overflow)) {
                 cur = first;
                 continue;
             }
@@ -417,34 +466,37 @@ __device__ __forceinline__ bool trace_scene_rt(bool ANY, bool COUNT, const Devic
             }
         }
         // pop the next entry that can still hold a counted hit
+        const int32_t limit = key_limit(t_best);
         for (;;) {
-            if (sp == 0) return ANY ? false : best_prim != HIT_NONE;
-            --sp;
-            if (st_t[sp] <= t_best) { cur = st_ref[sp]; break; }
+            if (st.empty()) return ANY ? false : best_prim != HIT_NONE;
+            const int2 e = st.pop();
+            if (e.x <= limit) { cur = e.y; break; }
         }
     }
 }
 
 template <bool ANY, bool COUNT>
-__device__ __forceinline__ bool trace_scene(const DeviceScene& S, const float4* __restrict__ snodes, uint32_t nsm,
-                                            f3 o, f3 d, float t_limit, float& t_best, int32_t& best_prim,
-                                            uint32_t& best_key, bool& overflow, TraceCounters& ctr) {
-    return trace_scene_rt(ANY, COUNT, S, snodes, nsm, o, d, t_limit, t_best, best_prim, best_key, overflow, ctr);
+__device__ __forceinline__ bool trace_scene(const DeviceScene& S, f3 o, f3 d, float t_limit, float& t_best,
+                                            int32_t& best_prim, uint32_t& best_key, bool& overflow,
+                                            TraceCounters& ctr) {
+    return trace_scene_rt(ANY, COUNT, S, o, d, t_limit, t_best, best_prim, best_key, overflow, ctr);
 }
 
 // ------------------------------------------------ resumable traversal ---
-// State of one ray's traversal, so a persistent warp can run a bounded
-// number of steps, hand finished lanes a new ray, and resume the others
-// (dynamic ray fetch).  Same tests and acceptance rules as trace_scene.
+// State of one ray's traversal, so a persistent warp can advance its lanes
+// step by step, hand finished lanes a new ray and resume the others.  Same
+// tests and acceptance rules as trace_scene.  `cur` is an inner node (>= 0), a
+// leaf's remaining primitives (< 0, as a child reference), or TRAV_IDLE.
+// Occlusion rays keep their limit in t_best, which never shrinks for them.
+constexpr int32_t TRAV_IDLE = 0x7fffffff;
 struct TravState {
-    f3 o, d, idir, ood;
-    float t_limit, t_best;
+    f3 o, d;
+    SlabRay r;
+    float t_best;
     int32_t best_prim;
     uint32_t best_key;
     int32_t cur;
-    int sp;
-    uint32_t guard;
-    bool done, hit;
+    bool hit;
     RefBoxCache cache;
 };
 
@@ -452,16 +504,11 @@ template <bool ANY>
 __device__ __forceinline__ void trav_init(const DeviceScene& S, TravState& s, f3 o, f3 d, float t_limit) {
     s.o = o;
     s.d = d;
-    s.idir = mk(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
-    s.ood = mk(o.x * s.idir.x, o.y * s.idir.y, o.z * s.idir.z);
-    s.t_limit = t_limit;
+    s.r = slab_ray(o, d);
     s.t_best = ANY ? t_limit : __int_as_float(0x7f800000);
     s.best_prim = HIT_NONE;
     s.best_key = 0xFFFFFFFFu;
-    s.cur = 0;
-    s.sp = 0;
-    s.guard = 2u * S.n_nodes + 64u;
-    s.done = false;
+    s.cur = S.n_nodes ? 0 : TRAV_IDLE;
     s.hit = false;
     s.cache.obj = -1;
     s.cache.ok = true;
@@ -471,158 +518,64 @@ __device__ __forceinline__ void trav_init(const DeviceScene& S, TravState& s, f3
         if (isect_plane(p0, p1, o, d, t)) {
             uint32_t key = __float_as_uint(p0.w);
             if (ANY) {
-                if (t <= t_limit) { s.hit = true; s.done = true; return; }
+                if (t <= t_limit) { s.hit = true; s.cur = TRAV_IDLE; return; }
             } else if (t < s.t_best || (t == s.t_best && key < s.best_key)) {
                 s.t_best = t; s.best_prim = prim_ref(3, i); s.best_key = key;
             }
         }
     }
-    if (S.n_nodes == 0) s.done = true;
 }
 
-// Pops the next entry that can still hold a counted hit; false when empty.
-// CHECK_T = false (occlusion rays): every entry can, none is skipped.
-template <bool CHECK_T = true>
-__device__ __forceinline__ bool trav_pop(TravState& s, const int32_t* st_ref, const float* st_t) {
-    if (!CHECK_T) {
-        if (s.sp == 0) return false;
-        s.cur = st_ref[--s.sp];
-        return true;
-    }
-    while (s.sp > 0) {
-        --s.sp;
-        if (st_t[s.sp] <= s.t_best) { s.cur = st_ref[s.sp]; return true; }
+// Accepts a candidate hit (t, key) of object obj (< 0: no finite box to ask):
+// true when an occlusion ray is blocked by it.
+template <bool ANY>
+__device__ __forceinline__ bool trav_accept(const DeviceScene& S, TravState& s, float t, uint32_t key, int32_t obj,
+                                            int32_t prim) {
+    if (ANY) return t <= s.t_best && (obj < 0 || s.cache.test(S, obj, s.o, s.d));
+    if ((t < s.t_best || (t == s.t_best && key < s.best_key)) && (obj < 0 || s.cache.test(S, obj, s.o, s.d))) {
+        s.t_best = t;
+        s.best_prim = prim;
+        s.best_key = key;
     }
     return false;
 }
 
-// Closest-hit test of the primitives of leaf v (packed start << 3 |
-// count - 1) against the ray of s, with trav_run's acceptance rules (the
-// packet traversal's leaf phase; trav_run keeps its own copy, which
-// compiles to faster any-hit code than a shared helper did).
-__device__ __forceinline__ void trav_leaf_closest(const DeviceScene& S, TravState& s, uint32_t v) {
+// Tests the primitives of leaf v (start << 3 | count - 1, one type per leaf)
+// against the ray of s; true when an occlusion ray is blocked.
+template <bool ANY, bool COUNT>
+__device__ __forceinline__ bool trav_leaf(const DeviceScene& S, TravState& s, uint32_t v, TraceCounters& ctr) {
     const uint32_t start = v >> 3, cnt = (v & 7u) + 1u;
-    const f3 o = s.o, d = s.d;
+    if (COUNT) ctr.tris += cnt;
+    float t;
     if (start < S.sphere_base) {
-        for (uint32_t k = 0; k < cnt; ++k) {
-            const uint32_t sl = start + k;
-            const float4* p = S.tris + 3 * (size_t)sl;
-            float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
-            float t;
-            if (!isect_tri(a, b, c, o, d, t)) continue;
-            const uint32_t key = __float_as_uint(a.w);
-            if ((t < s.t_best || (t == s.t_best && key < s.best_key)) && s.cache.test(S, __float_as_int(b.w), o, d)) {
-                s.t_best = t; s.best_prim = prim_ref(0, sl); s.best_key = key;
-            }
+        const float4* p = S.tris + 3 * (size_t)start;
+        for (uint32_t k = 0; k < cnt; ++k, p += 3) {
+            const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+            if (isect_tri(a, b, c, s.o, s.d, t) &&
+                trav_accept<ANY>(S, s, t, __float_as_uint(a.w), __float_as_int(b.w), prim_ref(0, start + k)))
+                return true;
         }
     } else if (start < S.quad_base) {
-        for (uint32_t k = 0; k < cnt; ++k) {
-            const uint32_t sl = start + k - S.sphere_base;
-            float4 s0 = __ldg(&S.spheres[2 * (size_t)sl]), s1 = __ldg(&S.spheres[2 * (size_t)sl + 1]);
-            float t;
-            if (!isect_sphere(s0, s1, o, d, t)) continue;
-            const uint32_t key = __float_as_uint(s0.w);
-            if ((t < s.t_best || (t == s.t_best && key < s.best_key)) && s.cache.test(S, __float_as_int(s1.z), o, d)) {
-                s.t_best = t; s.best_prim = prim_ref(1, sl); s.best_key = key;
-            }
+        const uint32_t first = start - S.sphere_base;
+        const float4* p = S.spheres + 2 * (size_t)first;
+        for (uint32_t k = 0; k < cnt; ++k, p += 2) {
+            const float4 a = __ldg(p), b = __ldg(p + 1);
+            if (isect_sphere(a, b, s.o, s.d, t) &&
+                trav_accept<ANY>(S, s, t, __float_as_uint(a.w), __float_as_int(b.z), prim_ref(1, first + k)))
+                return true;
         }
     } else {
-        for (uint32_t k = 0; k < cnt; ++k) {
-            const uint32_t sl = start + k - S.quad_base;
-            const float4* p = S.quads + 4 * (size_t)sl;
-            float4 q0 = __ldg(p), q1 = __ldg(p + 1), q2 = __ldg(p + 2), q3 = __ldg(p + 3);
-            float t;
-            if (!isect_quad(q0, q1, q2, q3, o, d, t)) continue;
-            const uint32_t key = __float_as_uint(q0.w);
-            if (t < s.t_best || (t == s.t_best && key < s.best_key)) {
-                s.t_best = t; s.best_prim = prim_ref(2, sl); s.best_key = key;
-            }
+        const uint32_t first = start - S.quad_base;
+        const float4* p = S.quads + 4 * (size_t)first;
+        for (uint32_t k = 0; k < cnt; ++k, p += 4) {
+            const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3);
+            // a quad's object box is infinite
+            if (isect_quad(a, b, c, d, s.o, s.d, t) &&
+                trav_accept<ANY>(S, s, t, __float_as_uint(a.w), -1, prim_ref(2, first + k)))
+                return true;
         }
     }
-}
-
-// Runs up to `rounds` rounds of (descend through inner nodes until a leaf,
-// test that leaf); lanes that are on inner nodes and lanes that are at a
-// leaf therefore execute their phases together (while-while).  Returns with
-// s.done set when the ray is finished.
-template <bool ANY, bool COUNT>
-__device__ __forceinline__ void trav_run(const DeviceScene& S, const float4* __restrict__ snodes, uint32_t nsm,
-                                         TravState& s, int32_t* st_ref, float* st_t, int rounds, bool& overflow,
-                                         TraceCounters& ctr) {
-    while (!s.done && rounds-- > 0) {
-        // inner phase
-        while (s.cur >= 0) {
-            if (--s.guard == 0u || (uint32_t)s.cur >= S.n_nodes) { overflow = true; s.done = true; return; }
-            float4 nb[7];
-            fetch_node(S, snodes, nsm, s.cur, nb);
-            if (COUNT) ctr.nodes++;
-            int32_t first;
-            if (visit4<!ANY>(nb, s.idir, s.ood, s.t_best, first, st_ref, st_t, s.sp, overflow)) {
-                s.cur = first;
-            } else if (!trav_pop<!ANY>(s, st_ref, st_t)) {
-                s.done = true;
-                return;
-            }
-        }
-        // leaf phase
-        const uint32_t v = ~(uint32_t)s.cur;
-        const uint32_t start = v >> 3, cnt = (v & 7u) + 1u;
-        const f3 o = s.o, d = s.d;
-        if (start < S.sphere_base) {
-            for (uint32_t k = 0; k < cnt; ++k) {
-                const uint32_t sl = start + k;
-                const float4* p = S.tris + 3 * (size_t)sl;
-                float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
-                if (COUNT) ctr.tris++;
-                float t;
-                if (!isect_tri(a, b, c, o, d, t)) continue;
-                const int32_t obj = __float_as_int(b.w);
-                if (ANY) {
-                    if (t <= s.t_limit && s.cache.test(S, obj, o, d)) { s.hit = true; s.done = true; return; }
-                } else {
-                    const uint32_t key = __float_as_uint(a.w);
-                    if ((t < s.t_best || (t == s.t_best && key < s.best_key)) && s.cache.test(S, obj, o, d)) {
-                        s.t_best = t; s.best_prim = prim_ref(0, sl); s.best_key = key;
-                    }
-                }
-            }
-        } else if (start < S.quad_base) {
-            for (uint32_t k = 0; k < cnt; ++k) {
-                const uint32_t sl = start + k - S.sphere_base;
-                float4 s0 = __ldg(&S.spheres[2 * (size_t)sl]), s1 = __ldg(&S.spheres[2 * (size_t)sl + 1]);
-                if (COUNT) ctr.tris++;
-                float t;
-                if (!isect_sphere(s0, s1, o, d, t)) continue;
-                const int32_t obj = __float_as_int(s1.z);
-                if (ANY) {
-                    if (t <= s.t_limit && s.cache.test(S, obj, o, d)) { s.hit = true; s.done = true; return; }
-                } else {
-                    const uint32_t key = __float_as_uint(s0.w);
-                    if ((t < s.t_best || (t == s.t_best && key < s.best_key)) && s.cache.test(S, obj, o, d)) {
-                        s.t_best = t; s.best_prim = prim_ref(1, sl); s.best_key = key;
-                    }
-                }
-            }
-        } else {
-            for (uint32_t k = 0; k < cnt; ++k) {
-                const uint32_t sl = start + k - S.quad_base;
-                const float4* p = S.quads + 4 * (size_t)sl;
-                float4 q0 = __ldg(p), q1 = __ldg(p + 1), q2 = __ldg(p + 2), q3 = __ldg(p + 3);
-                if (COUNT) ctr.tris++;
-                float t;
-                if (!isect_quad(q0, q1, q2, q3, o, d, t)) continue;
-                if (ANY) {
-                    if (t <= s.t_limit) { s.hit = true; s.done = true; return; }
-                } else {
-                    const uint32_t key = __float_as_uint(q0.w);
-                    if (t < s.t_best || (t == s.t_best && key < s.best_key)) {
-                        s.t_best = t; s.best_prim = prim_ref(2, sl); s.best_key = key;
-                    }
-                }
-            }
-        }
-        if (!trav_pop<!ANY>(s, st_ref, st_t)) { s.done = true; return; }
-    }
+    return false;
 }
 
 // ------------------------------------------------------ warp packets ---
@@ -642,25 +595,17 @@ __device__ __forceinline__ void trav_run(const DeviceScene& S, const float4* __r
 // when no lane hits a child; otherwise `first` is the child with the
 // nearest entry over the lanes and the other accepted children are pushed
 // far-to-near with each lane's own entry distance (INF where it missed).
-__device__ __forceinline__ bool packet_visit4(const float4* nb, f3 idir, f3 ood, float lim, int32_t& first,
-                                              int32_t* st_ref, float* st_t, int& sp, bool& overflow) {
+__device__ __forceinline__ bool packet_visit4(const float4* __restrict__ node, const SlabRay& sr, float lim,
+                                              int32_t& first, int32_t* st_ref, float* st_t, int& sp, bool& overflow) {
     const unsigned full = 0xffffffffu;
     const float INF = __int_as_float(0x7f800000);
-    const float lx[4] = {nb[0].x, nb[0].y, nb[0].z, nb[0].w}, hx[4] = {nb[1].x, nb[1].y, nb[1].z, nb[1].w};
-    const float ly[4] = {nb[2].x, nb[2].y, nb[2].z, nb[2].w}, hy[4] = {nb[3].x, nb[3].y, nb[3].z, nb[3].w};
-    const float lz[4] = {nb[4].x, nb[4].y, nb[4].z, nb[4].w}, hz[4] = {nb[5].x, nb[5].y, nb[5].z, nb[5].w};
-    int32_t r[4] = {__float_as_int(nb[6].x), __float_as_int(nb[6].y), __float_as_int(nb[6].z),
-                    __float_as_int(nb[6].w)};
+    const Slab4 s = slab4(node, sr, lim);
+    int32_t r[4] = {s.ref[0], s.ref[1], s.ref[2], s.ref[3]};
     float key[4];
     uint32_t wk[4];  // nearest entry over the lanes, as ordered bits (INF: no lane)
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const float x0 = __fmaf_rn(lx[k], idir.x, -ood.x), x1 = __fmaf_rn(hx[k], idir.x, -ood.x);
-        const float y0 = __fmaf_rn(ly[k], idir.y, -ood.y), y1 = __fmaf_rn(hy[k], idir.y, -ood.y);
-        const float z0 = __fmaf_rn(lz[k], idir.z, -ood.z), z1 = __fmaf_rn(hz[k], idir.z, -ood.z);
-        const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), 0.0f));
-        const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), lim));
-        key[k] = (tn <= tf && r[k] != BVH_EMPTY) ? tn : INF;
+        key[k] = s.hit[k] ? s.tn[k] : INF;
         // entry distances are >= 0 (a -0 clears to 0), so their bits order as the values
         wk[k] = __reduce_min_sync(full, __float_as_uint(key[k]) & 0x7fffffffu);
     }

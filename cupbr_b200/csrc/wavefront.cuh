@@ -33,61 +33,182 @@ __device__ __forceinline__ uint32_t claim_slot(bool want, uint32_t* counter) {
     return base + (uint32_t)__popc(mask & ((1u << lane_id()) - 1u));
 }
 
-// Persistent traversal over a queue with per-lane dynamic fetch: lanes whose
-// ray finished take the next rays of the queue (one atomicAdd per warp for
-// all of them) while the others resume their traversal, so a warp stays full
-// until the queue runs dry.  Entry i of the queue starts at q[stride * i]:
-// (origin, ANY ? t_limit : -), (direction, -).  ANY = false: closest hit,
-// ANY = true: occlusion up to t_limit.  done(i, state) runs once per ray.
-// The top smem_nodes BVH nodes are staged in shared memory (s_nodes).
-template <bool ANY, bool COUNT, bool NC = true, typename Done>
-__device__ __forceinline__ void persistent_trace(const DeviceScene& S, const float4* __restrict__ q, uint32_t stride,
-                                                 uint32_t count, uint32_t* fetch, uint32_t smem_nodes,
-                                                 float4* s_nodes, uint32_t* err_stack, uint64_t* stats, Done done) {
-    // a block that starts after the queue has been handed out (or on an empty
-    // queue) leaves before staging the top of the tree; the decision is the
-    // block's (the counter can move between two threads' reads)
-    if (!__syncthreads_or(*(volatile const uint32_t*)fetch < count)) return;
-    const uint32_t nsm = min(S.n_nodes, smem_nodes);
-    for (uint32_t i = threadIdx.x; i < nsm * BVH_NODE_F4; i += blockDim.x) s_nodes[i] = __ldg(&S.nodes[i]);
-    __syncthreads();
+// Traversal stack of a persistent lane: the first LEVELS entries in shared
+// memory, row by row over the block's threads (conflict free whatever the
+// lanes' depths; in local memory lanes at different depths touch a line
+// each), the rest in local memory.  Occlusion rays store references only.
+// 12 and 16 levels take 96 and 64 KB of an SM at 8 blocks of 128 threads;
+// with 8 the 1080p terrain took 46.1 ms instead of 45.4, with 6 47.4.
+template <bool ANY, int THREADS>
+struct LaneStack {
+    static constexpr int LEVELS = ANY ? 16 : 12;
+    static constexpr int ROW = THREADS * (ANY ? 4 : 8);  // bytes from one row to the next
+    static constexpr int NEAR = LEVELS * ROW;
+    static constexpr int FULL = CUPBR_STACK_SIZE * ROW;
+    char* base;  // this thread's entry of row 0
+    int sp;      // depth * ROW
+    int32_t far_ref[CUPBR_STACK_SIZE - LEVELS];
+    int32_t far_key[ANY ? 1 : CUPBR_STACK_SIZE - LEVELS];
+    __device__ __forceinline__ LaneStack(char* s_stack) : base(s_stack + threadIdx.x * (ANY ? 4 : 8)), sp(0) {}
+    __device__ __forceinline__ void clear() { sp = 0; }
+    __device__ __forceinline__ bool empty() const { return sp == 0; }
+    __device__ __forceinline__ void put(int at, int32_t key, int32_t ref) {
+        if (ANY) *reinterpret_cast<int32_t*>(base + at) = ref;
+        else *reinterpret_cast<int2*>(base + at) = make_int2(key, ref);
+    }
+    // room for three more entries in shared memory: put() them and raise sp
+    __device__ __forceinline__ bool near3() const { return sp <= NEAR - 3 * ROW; }
+    __device__ __forceinline__ void push(int32_t key, int32_t ref, bool& overflow) {
+        if (sp < NEAR) {
+            put(sp, key, ref);
+        } else if (sp < FULL) {
+            far_ref[(sp - NEAR) / ROW] = ref;
+            if (!ANY) far_key[(sp - NEAR) / ROW] = key;
+        } else {
+            overflow = true;
+            return;
+        }
+        sp += ROW;
+    }
+    __device__ __forceinline__ int2 pop() {
+        sp -= ROW;
+        if (sp < NEAR) {
+            if (ANY) return make_int2(0, *reinterpret_cast<const int32_t*>(base + sp));
+            return *reinterpret_cast<const int2*>(base + sp);
+        }
+        return make_int2(ANY ? 0 : far_key[(sp - NEAR) / ROW], far_ref[(sp - NEAR) / ROW]);
+    }
+};
+template <int THREADS>
+constexpr int TRACE_STACK_BYTES = LaneStack<false, THREADS>::NEAR;  // occlusion rays take 2/3 of it
 
+// Resumes the next stack entry that can still hold a counted hit.
+template <bool ANY, typename Stack>
+__device__ __forceinline__ void trav_pop(TravState& s, Stack& st) {
+    const int32_t limit = key_limit(s.t_best);
+    for (;;) {
+        if (st.empty()) { s.cur = TRAV_IDLE; return; }
+        const int2 e = st.pop();
+        if (ANY || e.x <= limit) { s.cur = e.y; return; }
+    }
+}
+
+constexpr int TRACE_NODE_STEPS = 3;
+constexpr int TRACE_REFILL = 12;
+
+// Queue entries a warp claims at once: a third of its share of what is left
+// of the queue, 32 to 128.  Large claims spare the one counter (32 at a time
+// doubled the shadow stage of a scene of 20 primitives), small ones keep the
+// warps' last rays even (128 to the end: 1080p terrain +1 %, 512: +8 %).
+__device__ __forceinline__ uint32_t trace_chunk(uint32_t count, uint32_t end, uint32_t warps) {
+    const uint32_t left = count - min(end, count);
+    return max(32u, min(128u, (left / (3u * warps)) & ~31u));
+}
+
+// Persistent traversal over a queue with per-lane dynamic fetch.  A warp's
+// lanes walk the tree in rounds of at most TRACE_NODE_STEPS node visits and
+// then one leaf: a bound on the visits, because a round that descends until
+// every lane holds a leaf runs as long as its slowest lane (9 of 32 lanes busy
+// on the 2M-triangle terrain's bounce rays; 13 with the bound).  Lanes whose
+// ray is done wait until TRACE_REFILL of them (or the whole warp) can hand in
+// their results and take the next rays together; the warp claims the queue in
+// chunks, so a refill rarely waits for an atomic.  Entry i of the queue starts
+// at q[stride * i]: (origin, ANY ? t_limit : -), (direction, -).  ANY = false:
+// closest hit, ANY = true: occlusion up to t_limit.  done(i, state) runs once
+// per ray.  s_stack: LaneStack<ANY, THREADS>::NEAR bytes of shared memory.
+//
+// Bound by issue slots and by the L1's load pipe (terrain, first bounce, B200:
+// 60 % and 65 % busy).  Measured on the 1080p terrain / the 512^2 Cornell box
+// (whole passes, one box): descent to a leaf by every lane and two such rounds
+// between refills 52.0 / 11.32 ms; this 45.1 / 10.65 ms; 2 or 4 node visits
+// 46.8 / 45.4 ms; a vote for the phase with more lanes before every step
+// 47.1 / 12.2 ms (15 lanes busy, but the votes cost what they gain); one
+// primitive per round instead of a leaf 50.7 / 13.4 ms; refills at 4 idle
+// lanes 46.2 ms.
+template <bool ANY, bool COUNT, int THREADS, bool NC = true, typename Done>
+__device__ __forceinline__ void persistent_trace(const DeviceScene& S, const float4* __restrict__ q, uint32_t stride,
+                                                 uint32_t count, uint32_t* fetch, char* s_stack, uint32_t* err_stack,
+                                                 uint64_t* stats, Done done) {
     const unsigned full = 0xffffffffu;
     const uint32_t lane = lane_id();
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    // a well-formed tree visits every node at most once per ray, and a round
+    // advances every lane that is on a ray
+    const uint64_t guard = 4ull * S.n_nodes + 64u + S.n_tris + S.n_spheres + S.n_quads;
     TravState s;
-    int32_t st_ref[CUPBR_STACK_SIZE];
-    float st_t[CUPBR_STACK_SIZE];
+    s.cur = TRAV_IDLE;
+    LaneStack<ANY, THREADS> st(s_stack);
     TraceCounters tc;
-    bool overflow = false, have = false, exhausted = false;
-    uint32_t idx = 0;
+    bool overflow = false, have = false;
+    uint32_t idx = 0, next = 0, end = 0;  // next, end: the warp's chunk of the queue
+    uint64_t steps = 0;
     for (;;) {
-        const bool want = !have && !exhausted;
-        const unsigned m = __ballot_sync(full, want);
-        if (m) {
-            const int leader = __ffs(m) - 1;
-            uint32_t base = 0;
-            if ((int)lane == leader) base = atomicAdd(fetch, (uint32_t)__popc(m));
-            base = __shfl_sync(full, base, leader);
-            if (want) {
-                idx = base + (uint32_t)__popc(m & ((1u << lane) - 1u));
+        const unsigned m_idle = __ballot_sync(full, s.cur == TRAV_IDLE);
+        if (m_idle == full || (__popc(m_idle) >= TRACE_REFILL && next < count)) {
+            // finished lanes hand in their results and take the next rays
+            const bool idle = s.cur == TRAV_IDLE;
+            if (idle && have) {
+                have = false;
+                done(idx, s);
+            }
+            if (next >= count) {
+                if (m_idle == full) break;
+                continue;
+            }
+            const uint32_t n = (uint32_t)__popc(m_idle);
+            uint32_t fresh = 0, chunk = 0;
+            if (next + n > end) {
+                chunk = trace_chunk(count, end, warps);
+                if (lane == 0) fresh = atomicAdd(fetch, chunk);
+                fresh = __shfl_sync(full, fresh, 0);
+            }
+            if (idle) {
+                idx = next + (uint32_t)__popc(m_idle & ((1u << lane) - 1u));
+                if (idx >= end) idx = fresh + (idx - end);
                 if (idx < count) {
                     const float4 q0 = qload<NC>(&q[stride * (size_t)idx]);
                     const float4 q1 = qload<NC>(&q[stride * (size_t)idx + 1]);
                     trav_init<ANY>(S, s, xyz(q0), xyz(q1), ANY ? q0.w : 0.0f);
+                    st.clear();
                     have = true;
+                }
+            }
+            if (next + n > end) {
+                next = fresh + (next + n - end);
+                end = fresh + chunk;
+            } else {
+                next += n;
+            }
+            steps = 0;
+            continue;
+        }
+        if (++steps > guard) {  // a malformed tree: report and stop
+            overflow = true;
+            s.cur = TRAV_IDLE;
+            continue;
+        }
+#pragma unroll
+        for (int u = 0; u < TRACE_NODE_STEPS; ++u) {
+            if (s.cur >= 0 && s.cur != TRAV_IDLE) {
+                if ((uint32_t)s.cur >= S.n_nodes) {  // corrupt reference
+                    overflow = true;
+                    s.cur = TRAV_IDLE;
                 } else {
-                    exhausted = true;
+                    if (COUNT) tc.nodes++;
+                    int32_t first;
+                    if (visit4<ANY>(S.nodes + BVH_NODE_F4 * (size_t)s.cur, s.r, s.t_best, first, st, overflow))
+                        s.cur = first;
+                    else
+                        trav_pop<ANY>(s, st);
                 }
             }
         }
-        if (!__ballot_sync(full, have)) break;
-        if (have) {
-            // two descent + leaf rounds between refills (measured best: one round
-            // pays the refill too often, four or more let finished lanes idle)
-            trav_run<ANY, COUNT>(S, s_nodes, nsm, s, st_ref, st_t, 2, overflow, tc);
-            if (s.done) {
-                have = false;
-                done(idx, s);
+        if (s.cur < 0) {
+            if (trav_leaf<ANY, COUNT>(S, s, ~(uint32_t)s.cur, tc)) {
+                s.hit = true;
+                s.cur = TRAV_IDLE;
+            } else {
+                trav_pop<ANY>(s, st);
             }
         }
     }
@@ -120,13 +241,31 @@ __device__ __forceinline__ uint32_t slot_pixel(uint32_t s, uint32_t w, uint32_t 
     return h4 * w + (s - rw * h4);
 }
 
+// Queue slot of a wavefront of `frames` frames -> (frame, pixel): tile by tile,
+// each tile's 32 pixels in every frame before the next tile's, so the rays in
+// flight at a time start from a small part of the screen and share the tree's
+// nodes in the caches; the strips the tiles leave follow frame by frame.
+__device__ __forceinline__ void slot_path(uint32_t s, uint32_t w, uint32_t h, uint32_t frames, uint32_t& fr,
+                                          uint32_t& pixel) {
+    const uint32_t tiled = (w >> 3) * 8u * (h & ~3u), pixels = w * h;
+    if (s < tiled * frames) {
+        const uint32_t t = s / (32u * frames), r = s - t * 32u * frames;
+        fr = r >> 5;
+        pixel = slot_pixel(32u * t + (r & 31u), w, h);
+    } else {
+        const uint32_t strip = pixels - tiled;
+        s -= tiled * frames;
+        fr = s / strip;
+        pixel = slot_pixel(tiled + (s - fr * strip), w, h);
+    }
+}
+
 // Closest hits of one warp's 32 rays walked as a packet (packet_visit4):
 // every lane of the warp calls it together; a lane with valid = false takes
 // part in the walk but accepts no box.  On return s holds the lane's hit as
 // trav_run leaves it (t_best, best_prim, best_key).
-__device__ __forceinline__ void packet_closest(const DeviceScene& S, const float4* s_nodes, uint32_t nsm, f3 o, f3 d,
-                                               bool valid, TravState& s, int32_t* st_ref, float* st_t,
-                                               bool& overflow) {
+__device__ __forceinline__ void packet_closest(const DeviceScene& S, f3 o, f3 d, bool valid, TravState& s,
+                                               int32_t* st_ref, float* st_t, bool& overflow) {
     trav_init<false>(S, s, o, d, 0.0f);
     // a lane past the end of the queue accepts no box (t_f <= -1 < t_n)
     if (!valid) s.t_best = -1.0f;
@@ -137,13 +276,14 @@ __device__ __forceinline__ void packet_closest(const DeviceScene& S, const float
     while (live) {
         if (cur >= 0) {
             if (--guard == 0u || (uint32_t)cur >= S.n_nodes) { overflow = true; break; }
-            float4 nb[7];
-            fetch_node(S, s_nodes, nsm, cur, nb);
             int32_t first;
-            if (packet_visit4(nb, s.idir, s.ood, s.t_best, first, st_ref, st_t, sp, overflow)) cur = first;
+            if (packet_visit4(S.nodes + BVH_NODE_F4 * (size_t)cur, s.r, s.t_best, first, st_ref, st_t, sp,
+                              overflow))
+                cur = first;
             else live = packet_pop(s.t_best, st_ref, st_t, sp, cur);
         } else {
-            if (valid) trav_leaf_closest(S, s, ~(uint32_t)cur);
+            TraceCounters tc;
+            if (valid) trav_leaf<false, false>(S, s, ~(uint32_t)cur, tc);
             live = packet_pop(s.t_best, st_ref, st_t, sp, cur);
         }
     }
@@ -157,13 +297,7 @@ __device__ __forceinline__ void packet_closest(const DeviceScene& S, const float
 // on.  No traversal counters (instrumented frames use persistent_trace).
 template <bool NC = true, typename Done>
 __device__ __forceinline__ void packet_trace(const DeviceScene& S, const float4* __restrict__ q, uint32_t stride,
-                                             uint32_t count, uint32_t* fetch, uint32_t smem_nodes, float4* s_nodes,
-                                             uint32_t* err_stack, Done done) {
-    if (!__syncthreads_or(*(volatile const uint32_t*)fetch < count)) return;  // as persistent_trace
-    const uint32_t nsm = min(S.n_nodes, smem_nodes);
-    for (uint32_t i = threadIdx.x; i < nsm * BVH_NODE_F4; i += blockDim.x) s_nodes[i] = __ldg(&S.nodes[i]);
-    __syncthreads();
-
+                                             uint32_t count, uint32_t* fetch, uint32_t* err_stack, Done done) {
     const unsigned full = 0xffffffffu;
     const uint32_t lane = lane_id();
     int32_t st_ref[CUPBR_STACK_SIZE];
@@ -182,7 +316,7 @@ __device__ __forceinline__ void packet_trace(const DeviceScene& S, const float4*
             d = xyz(qload<NC>(&q[stride * (size_t)idx + 1]));
         }
         TravState s;
-        packet_closest(S, s_nodes, nsm, o, d, valid, s, st_ref, st_t, overflow);
+        packet_closest(S, o, d, valid, s, st_ref, st_t, overflow);
         if (valid) done(idx, s);
     }
     if (overflow) atomicAdd(err_stack, 1u);
