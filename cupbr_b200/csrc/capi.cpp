@@ -356,11 +356,9 @@ struct cupbr_postprocessor_s {
     const float* hdr = nullptr;
     uint32_t w = 0, h = 0;
     float* out = nullptr;
-    float* half = nullptr;
     cudaStream_t stream = nullptr;
     ~cupbr_postprocessor_s() {
         if (out) cudaFree(out);
-        if (half) cudaFree(half);
     }
 };
 
@@ -1394,10 +1392,8 @@ int cupbr_postprocessor_register_image(cupbr_postprocessor_t p, const float* hdr
     if (!p || !hdr) return fail(CUPBR_ERR_ARG, "null argument");
     if (w < 2 || h < 2) return fail(CUPBR_ERR_ARG, "bloom needs an image of at least 2x2 pixels");
     if (p->out) cudaFree(p->out);
-    if (p->half) cudaFree(p->half);
-    p->out = p->half = nullptr;
+    p->out = nullptr;
     CUPBR_CHECK_CUDA(dev_alloc(&p->out, sizeof(float) * 3 * (size_t)w * h));
-    CUPBR_CHECK_CUDA(dev_alloc(&p->half, sizeof(float) * 3 * (size_t)(w / 2) * (h / 2)));
     p->hdr = hdr;
     p->w = w;
     p->h = h;
@@ -1412,7 +1408,7 @@ int cupbr_postprocessor_bloom(cupbr_postprocessor_t p, const float th[4]) {
     NvtxRange nvtx_("cupbr_postprocessor_bloom");
     if (!p || !th) return fail(CUPBR_ERR_ARG, "null argument");
     if (!p->hdr) return fail(CUPBR_ERR_STATE, "no image registered");
-    CUPBR_CHECK_CUDA(launch_bloom(p->hdr, p->w, p->h, th, p->half, p->out, nullptr, 0, 0.0f, p->stream));
+    CUPBR_CHECK_CUDA(launch_bloom(p->hdr, p->w, p->h, th, p->out, nullptr, 0, 0.0f, p->stream));
     return CUPBR_OK;
 }
 int cupbr_postprocessor_bloom_tonemap(cupbr_postprocessor_t p, const float th[4], int32_t type, float exposure,
@@ -1421,7 +1417,7 @@ int cupbr_postprocessor_bloom_tonemap(cupbr_postprocessor_t p, const float th[4]
     if (!p || !th || !rgba) return fail(CUPBR_ERR_ARG, "null argument");
     if (!p->hdr) return fail(CUPBR_ERR_STATE, "no image registered");
     if (type != CUPBR_REINHARD && type != CUPBR_GAMMA) return fail(CUPBR_ERR_ARG, "unknown tone mapping type");
-    CUPBR_CHECK_CUDA(launch_bloom(p->hdr, p->w, p->h, th, p->half, nullptr, rgba, type, exposure, p->stream));
+    CUPBR_CHECK_CUDA(launch_bloom(p->hdr, p->w, p->h, th, nullptr, rgba, type, exposure, p->stream));
     return CUPBR_OK;
 }
 // Bloom for callers that cannot allocate device memory: the level-1 scratch

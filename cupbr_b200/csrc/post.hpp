@@ -21,15 +21,14 @@ cudaError_t ensure_tone_levels(cudaStream_t st);
 // Synchronizes the stream.
 cudaError_t verify_tone_levels(unsigned long long mismatches[3], uint32_t flagged[3], cudaStream_t st);
 
-// PostProcessor::bloom (pyramid depth 6 semantics).  scratch_half holds
-// (w/2) * (h/2) * 3 floats.  With rgba == nullptr the HDR result goes to
-// `out`; otherwise the result is tone-mapped into rgba and `out` is unused.
-// Requires w >= 2 and h >= 2.
-cudaError_t launch_bloom(const float* hdr, uint32_t w, uint32_t h, const float th[4], float* scratch_half, float* out,
-                         uint8_t* rgba, int type, float exposure, cudaStream_t st);
+// PostProcessor::bloom (pyramid depth 6 semantics).  With rgba == nullptr the
+// HDR result goes to `out`; otherwise the result is tone-mapped into rgba and
+// `out` is unused.  Requires w >= 2 and h >= 2 and an output apart from hdr.
+cudaError_t launch_bloom(const float* hdr, uint32_t w, uint32_t h, const float th[4], float* out, uint8_t* rgba,
+                         int type, float exposure, cudaStream_t st);
 
-// Bloom with its level-1 scratch in a fixed device array owned by the
-// library (no allocation).  At most BLOOM_NOALLOC_MAX_HALF_PIXELS level-1
+// Bloom that allocates nothing; an output that lies over its input gets its
+// level-1 scratch in a fixed device array owned by the library.  At most BLOOM_NOALLOC_MAX_HALF_PIXELS level-1
 // pixels, i.e. (w/2) * (h/2) <= 1048576 (inputs up to 2048 x 2048); the
 // caller checks the size.  Calls whose work overlaps on the GPU share the
 // array and race.
