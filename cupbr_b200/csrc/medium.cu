@@ -181,21 +181,22 @@ __device__ __forceinline__ void params_end(const float* s_params, uint32_t np_sm
         if (s_params[k] != 0.0f) atomicAdd(&g_params[k], s_params[k]);
 }
 
-// TracingDetail.h:15-30 camera rays (as the path tracer's k_camera) into ray
-// queue 0: (origin, path), (direction, seed), (1, pending Lambert object + 1
+// TracingDetail.h:15-30 camera rays (as the path tracer's k_camera, in its slot
+// order: slot_path) into ray queue 0: (origin, path), (direction, seed), (1, pending Lambert object + 1
 // = 0).  RENDER / LSUM clear the path's radiance sum; ADJOINT keeps it (it
 // is the L_rem of the replay) and enqueues only paths whose pixel has a
 // nonzero dLoss/dI.
 template <int MODE>
 __global__ void k_medium_camera(MediumParams P, MediumBatch B, Workspace W, double* __restrict__ lsum,
                                 const float* __restrict__ grad_img) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     bool push = false;
     f3 o = P.cam_pos, d = mk(0.0f, 0.0f, 1.0f);
-    uint32_t seed = 0;
-    if (p < B.n_paths) {
-        const uint32_t fr = p / B.pixels;
-        const uint32_t tid = p - fr * B.pixels;
+    uint32_t seed = 0, p = 0;
+    if (i < B.n_paths) {
+        uint32_t fr, tid;
+        slot_path(i, P.width, P.height, B.frames, fr, tid);
+        p = fr * B.pixels + tid;
         seed = tea4(tid, B.sample0 + fr);
         const uint32_t py = tid / P.width, px = tid - P.width * py;
         const float jx = rnd(seed);
@@ -212,7 +213,15 @@ __global__ void k_medium_camera(MediumParams P, MediumBatch B, Workspace W, doub
             else lsum[3 * (size_t)p] = lsum[3 * (size_t)p + 1] = lsum[3 * (size_t)p + 2] = 0.0;
         }
     }
-    const uint32_t slot = claim_slot(push, &W.ctr[CTR_RAYS + 0]);
+    uint32_t slot = i;
+    if (MODE == ADJOINT) {
+        __shared__ BlockClaim<1, 8> s_claim;
+        uint32_t slots[1];
+        s_claim({push}, {&W.ctr[CTR_RAYS + 0]}, slots);
+        slot = slots[0];
+    } else if (i == 0) {
+        W.ctr[CTR_RAYS + 0] = B.n_paths;
+    }
     if (push) {
         float4* q = W.rays[0] + 3 * (size_t)slot;
         q[0] = f4(o, __uint_as_float(p));
@@ -390,11 +399,10 @@ __global__ void __launch_bounds__(256) k_medium_scatter(DeviceScene S, MediumPar
     const uint32_t count = W.ctr[CTR_MVERT + depth];
     float4* __restrict__ qn = W.rays[(depth + 1) & 1];
     const bool last = depth + 1 >= P.max_depth;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t nl = S.n_lights;
-    for (uint32_t i0 = warp * 32u; i0 < count; i0 += nwarps * 32u) {
-        const uint32_t i = i0 + lane_id();
+    __shared__ BlockClaim<2, 8> s_claim;
+    for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < count; i0 += gridDim.x * blockDim.x) {
+        const uint32_t i = i0 + threadIdx.x;
         bool push_sh = false, push_ext = false;
         float4 sh0, sh1, sh2, shx, ex0, ex1, ex2;
         if (i < count) {
@@ -424,7 +432,9 @@ __global__ void __launch_bounds__(256) k_medium_scatter(DeviceScene S, MediumPar
                 ex2 = f4(beta, 0.0f);
             }
         }
-        const uint32_t ss = claim_slot(push_sh, &W.ctr[CTR_SHADOW + depth]);
+        uint32_t slot[2];
+        s_claim({push_sh, push_ext}, {&W.ctr[CTR_SHADOW + depth], &W.ctr[CTR_RAYS + depth + 1]}, slot);
+        const uint32_t ss = slot[0], es = slot[1];
         if (push_sh) {
             float4* e = W.shadow + 3 * (size_t)ss;
             e[0] = sh0;
@@ -432,7 +442,6 @@ __global__ void __launch_bounds__(256) k_medium_scatter(DeviceScene S, MediumPar
             e[2] = sh2;
             shadow_aux[ss] = shx;
         }
-        const uint32_t es = claim_slot(push_ext, &W.ctr[CTR_RAYS + depth + 1]);
         if (push_ext) {
             float4* e = qn + 3 * (size_t)es;
             e[0] = ex0;
@@ -458,11 +467,10 @@ __global__ void __launch_bounds__(256, 3) k_medium_surface(DeviceScene S, Medium
     const uint32_t count = W.ctr[CTR_SVERT + depth];
     float4* __restrict__ qn = W.rays[(depth + 1) & 1];
     const bool last = depth + 1 >= P.max_depth;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t nl = S.n_lights;
-    for (uint32_t i0 = warp * 32u; i0 < count; i0 += nwarps * 32u) {
-        const uint32_t i = i0 + lane_id();
+    __shared__ BlockClaim<2, 8> s_claim;
+    for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < count; i0 += gridDim.x * blockDim.x) {
+        const uint32_t i = i0 + threadIdx.x;
         bool push_sh = false, push_ext = false;
         float4 sh0, sh1, sh2, shx, ex0, ex1, ex2;
         if (i < count) {
@@ -523,7 +531,9 @@ __global__ void __launch_bounds__(256, 3) k_medium_surface(DeviceScene S, Medium
                 }
             }
         }
-        const uint32_t ss = claim_slot(push_sh, &W.ctr[CTR_SHADOW + depth]);
+        uint32_t slot[2];
+        s_claim({push_sh, push_ext}, {&W.ctr[CTR_SHADOW + depth], &W.ctr[CTR_RAYS + depth + 1]}, slot);
+        const uint32_t ss = slot[0], es = slot[1];
         if (push_sh) {
             float4* e = W.shadow + 3 * (size_t)ss;
             e[0] = sh0;
@@ -531,7 +541,6 @@ __global__ void __launch_bounds__(256, 3) k_medium_surface(DeviceScene S, Medium
             e[2] = sh2;
             shadow_aux[ss] = shx;
         }
-        const uint32_t es = claim_slot(push_ext, &W.ctr[CTR_RAYS + depth + 1]);
         if (push_ext) {
             float4* e = qn + 3 * (size_t)es;
             e[0] = ex0;

@@ -152,8 +152,11 @@ __device__ __forceinline__ uint32_t vol_class(const DeviceScene& S, float2 h) {
 }
 
 // The body of the reference's depth loop (VolumeRenderer.cu:88-310) for one
-// queue entry.
-__global__ void __launch_bounds__(256, 2) k_vol_shade(const __grid_constant__ DeviceScene S, PTFrame F, Workspace W,
+// queue entry.  4 blocks per SM (64 registers, with spills): latency bound, so
+// the warps weigh more than the spills (512 x 512 x 32 frames, 5 depths, B200: 2
+// blocks 6.4 ms, 3 5.9, 4 5.6, 5 5.9; paths inside a mesh apart from those inside
+// a sphere 5.6 -> 5.3).
+__global__ void __launch_bounds__(256, 4) k_vol_shade(const __grid_constant__ DeviceScene S, PTFrame F, Workspace W,
                                                       uint32_t depth) {
     const uint32_t n_out = W.ctr[CTR_RAYS + depth], n_in = W.ctr[CTR_VOL_INSIDE + depth];
     const uint32_t n = n_out + n_in;
@@ -165,16 +168,23 @@ __global__ void __launch_bounds__(256, 2) k_vol_shade(const __grid_constant__ De
     const f3 scene_ss = xyz(S.vol_sigma_s), scene_sa = xyz(S.vol_sigma_a);
     const float scene_g = S.vol_sigma_s.w;
     // each chunk of 256 entries is shaded in class order (misses, VOLUME
-    // interfaces, diffuse, GGX, mirror / glass, paths inside an object), so
-    // most warps run one branch of the bounce
-    constexpr uint32_t NC = 6;
+    // interfaces, diffuse, GGX, mirror / glass, paths inside an object, those
+    // inside a mesh, whose triangles they test one by one), so most warps run one
+    // branch of the bounce
+    constexpr uint32_t NC = 7;
     __shared__ uint32_t s_cnt[8][NC];
     __shared__ uint32_t s_idx[256];
+    __shared__ BlockClaim<3, 8> s_claim;
     const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
     for (uint32_t c0 = blockIdx.x * 256u; c0 < n; c0 += gridDim.x * 256u) {
         const uint32_t mine = c0 + threadIdx.x;
         uint32_t cls = NC;  // past the end
-        if (mine < n) cls = mine >= n_out ? NC - 1 : vol_class(S, __ldg(&W.hits[mine]));
+        if (mine < n_out) {
+            cls = vol_class(S, __ldg(&W.hits[mine]));
+        } else if (mine < n) {
+            const uint32_t in = __float_as_uint(__ldg(&q[3 * (size_t)(F.n_paths - 1 - (mine - n_out)) + 2]).w);
+            cls = __ldg(&S.obj_info[in - 1u]).x == 4 ? NC - 1 : NC - 2;
+        }
         uint32_t rank = 0;
 #pragma unroll
         for (uint32_t k = 0; k < NC; ++k) {
@@ -277,7 +287,7 @@ __global__ void __launch_bounds__(256, 2) k_vol_shade(const __grid_constant__ De
                                 }
                                 const f3 sst = scene_sa + scene_ss;
                                 const f3 c = nl * vexp(-1.0f * sst * fminf(dist, 100000000.0f)) * att * lrad * rw;
-                                push_sh = true;
+                                push_sh = !is_zero(c);  // a zero term changes no sum
                                 sh0 = f4(so, dist);
                                 sh1 = f4(normalize(ldir), __uint_as_float(pid));
                                 sh2 = f4(c, 0.0f);
@@ -315,7 +325,7 @@ __global__ void __launch_bounds__(256, 2) k_vol_shade(const __grid_constant__ De
                             const f3 c = nl * fmaxf(0.0f, dot(g.N, ldir)) *
                                          vexp(-1.0f * (vss + vsa) * fminf(dist, 100000000.0f)) *
                                          brdf(m, inc, ldir, g.N) * lrad * rw;
-                            push_sh = true;
+                            push_sh = !is_zero(c);  // a zero term changes no sum
                             sh0 = f4(g.P + 0.001f * ldir, dist);
                             sh1 = f4(normalize(ldir), __uint_as_float(pid));
                             sh2 = f4(c, 0.0f);
@@ -344,9 +354,10 @@ __global__ void __launch_bounds__(256, 2) k_vol_shade(const __grid_constant__ De
                 }
             }
         }
-        const uint32_t ss = claim_slot(push_sh, &W.ctr[CTR_SHADOW + depth]);
-        const uint32_t so = claim_slot(push_next && !next_inside, &W.ctr[CTR_RAYS + depth + 1]);
-        const uint32_t si = claim_slot(push_next && next_inside, &W.ctr[CTR_VOL_INSIDE + depth + 1]);
+        uint32_t slot[3];
+        s_claim({push_sh, push_next && !next_inside, push_next && next_inside},
+                {&W.ctr[CTR_SHADOW + depth], &W.ctr[CTR_RAYS + depth + 1], &W.ctr[CTR_VOL_INSIDE + depth + 1]}, slot);
+        const uint32_t ss = slot[0], so = slot[1], si = slot[2];
         if (push_sh) {
             float4* e = W.shadow + 3 * (size_t)ss;
             e[0] = sh0;
@@ -432,7 +443,10 @@ __global__ void k_gd_camera_shift(PTFrame F, Workspace W, uint32_t n_int, const 
         want = (valid[v] & 1ull) != 0ull;
         W.radiance[n_base + 4u * v + k - 1u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
-    const uint32_t slot = claim_slot(want, &W.ctr[CTR_RAYS + 0]);
+    __shared__ BlockClaim<1, 8> s_claim;
+    uint32_t slots[1];
+    s_claim({want}, {&W.ctr[CTR_RAYS + 0]}, slots);
+    const uint32_t slot = slots[0];
     if (!want) return;
     f3 o, d;
     uint32_t seed;
@@ -444,9 +458,10 @@ __global__ void k_gd_camera_shift(PTFrame F, Workspace W, uint32_t n_int, const 
 }
 
 // The body of collect_radiance's depth loop (GradientDomain.cu:110-158)
-// for one queue entry.
+// for one queue entry.  4 blocks per SM as k_vol_shade (both kernels of 512 x 512
+// x 8 frames: 2 blocks 2.25 ms, 3 1.87, 4 1.59, 5 1.89).
 template <bool SHIFT>
-__global__ void __launch_bounds__(256, 2) k_gd_shade(const __grid_constant__ DeviceScene S, PTFrame F, Workspace W,
+__global__ void __launch_bounds__(256, 4) k_gd_shade(const __grid_constant__ DeviceScene S, PTFrame F, Workspace W,
                                                      uint32_t depth, uint32_t n_base, uint64_t* __restrict__ valid) {
     const uint32_t n = W.ctr[CTR_RAYS + depth];
     const float4* __restrict__ q = W.rays[depth & 1];
@@ -454,6 +469,7 @@ __global__ void __launch_bounds__(256, 2) k_gd_shade(const __grid_constant__ Dev
     const bool last = depth + 1 >= F.max_depth;
     const uint32_t L = S.n_lights, use_env = S.env_w > 0 ? 1u : 0u;
     const float nl = (float)(L + use_env);
+    __shared__ BlockClaim<2, 8> s_claim;
     for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
         const uint32_t i = i0 + threadIdx.x;
         bool push_sh = false, push_next = false;
@@ -496,7 +512,7 @@ __global__ void __launch_bounds__(256, 2) k_gd_shade(const __grid_constant__ Dev
                     float dist;
                     const f3 lrad = sample_nee(S, m, seed, g.P, inc, g.N, ldir, dist);
                     const f3 c = nl * fmaxf(0.0f, dot(g.N, ldir)) * brdf(m, inc, ldir, g.N) * lrad * rw;
-                    push_sh = true;
+                    push_sh = !is_zero(c);  // a zero term changes no sum
                     sh0 = f4(g.P + 0.001f * ldir, dist);
                     sh1 = f4(normalize(ldir), __uint_as_float(pid));
                     sh2 = f4(c, 0.0f);
@@ -516,8 +532,9 @@ __global__ void __launch_bounds__(256, 2) k_gd_shade(const __grid_constant__ Dev
                 }
             }
         }
-        const uint32_t ss = claim_slot(push_sh, &W.ctr[CTR_SHADOW + depth]);
-        const uint32_t sn = claim_slot(push_next, &W.ctr[CTR_RAYS + depth + 1]);
+        uint32_t slot[2];
+        s_claim({push_sh, push_next}, {&W.ctr[CTR_SHADOW + depth], &W.ctr[CTR_RAYS + depth + 1]}, slot);
+        const uint32_t ss = slot[0], sn = slot[1];
         if (push_sh) {
             float4* e = W.shadow + 3 * (size_t)ss;
             e[0] = sh0;

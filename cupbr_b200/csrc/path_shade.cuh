@@ -238,11 +238,18 @@ __device__ __forceinline__ void shade_stage(const DeviceScene& S, const PTFrame&
     // diffuse, GGX, delta), so most warps run one BSDF's code
     __shared__ uint32_t s_cnt[8][4];
     __shared__ uint32_t s_idx[256];
+    constexpr int QUEUES = CACHE ? 3 : 2;
+    __shared__ BlockClaim<QUEUES, 8> s_claim;
     const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
     const unsigned full = 0xffffffffu;
 
     for (uint32_t c0 = blockIdx.x * 256u; c0 < count; c0 += gridDim.x * 256u) {
         const uint32_t mine = c0 + threadIdx.x;
+        if (NC && c0 + gridDim.x * 256u < count) {
+            const uint32_t n0 = c0 + gridDim.x * 256u, left = min(256u, count - n0);
+            prefetch_block(q + 3 * (size_t)n0, 48u * left);
+            prefetch_block(W.hits + n0, 8u * left);
+        }
         uint32_t cls = 4;  // past the end
         if (mine < count) cls = shade_class(S, NC ? W.hits[mine] : __ldcg(&W.hits[mine]));
         uint32_t rank = 0;
@@ -270,24 +277,29 @@ __device__ __forceinline__ void shade_stage(const DeviceScene& S, const PTFrame&
             const float4 q2 = qload<NC>(&q[3 * (size_t)i + 2]);
             shade_one<CACHE, PHYS, NC>(S, F, W, C, depth, q0, q1, q2, NC ? W.hits[i] : __ldcg(&W.hits[i]), so);
         }
-        uint32_t ss = claim_slot(so.sh, &W.ctr[CTR_SHADOW + depth]);
+        uint32_t slot[QUEUES];
+        if constexpr (CACHE) {
+            s_claim({so.sh, so.ext, so.q}, {&W.ctr[CTR_SHADOW + depth], &W.ctr[CTR_RAYS + depth + 1], C.n_queries},
+                    slot);
+        } else {
+            s_claim({so.sh, so.ext}, {&W.ctr[CTR_SHADOW + depth], &W.ctr[CTR_RAYS + depth + 1]}, slot);
+        }
         if (so.sh) {
-            float4* e = W.shadow + 3 * (size_t)ss;
+            float4* e = W.shadow + 3 * (size_t)slot[0];
             e[0] = so.s0; e[1] = so.s1; e[2] = so.s2;
         }
-        uint32_t es = claim_slot(so.ext, &W.ctr[CTR_RAYS + depth + 1]);
         if (so.ext) {
-            float4* e = qn + 3 * (size_t)es;
+            float4* e = qn + 3 * (size_t)slot[1];
             e[0] = so.e0; e[1] = so.e1; e[2] = so.e2;
         }
-        if (CACHE) {
-            uint32_t qs = claim_slot(so.q, C.n_queries);
+        if constexpr (CACHE) {
             if (so.q) {
 #pragma unroll
-                for (int k = 0; k < (int)RC_REC; ++k) C.queries[(size_t)k * C.query_stride + qs] = so.cq[k];
+                for (int k = 0; k < (int)RC_REC; ++k) C.queries[(size_t)k * C.query_stride + slot[2]] = so.cq[k];
             }
         }
-        __syncthreads();  // s_cnt / s_idx of the next chunk
+        // s_claim's last barrier also frees s_cnt and s_idx for the next chunk;
+        // its own counts are read before the next chunk's first barrier
     }
 }
 

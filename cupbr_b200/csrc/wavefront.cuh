@@ -93,6 +93,58 @@ __device__ __forceinline__ void trav_pop(TravState& s, Stack& st) {
     }
 }
 
+// Asks L2 for the bytes [p, p + bytes) that the block reads in its next chunk
+// (p 16-byte aligned): the threads take a 128-byte line each.  The stage
+// kernels read queues that the traversal wrote through to DRAM, at the head of
+// a chain of dependent loads.
+__device__ __forceinline__ void prefetch_block(const void* p, uint32_t bytes) {
+    const uint32_t at = threadIdx.x * 128u;
+    if (at < bytes)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(static_cast<const char*>(p) + at)));
+}
+
+// Queue slots for a block: lanes with want[k] set get consecutive slots of
+// queue k, one atomicAdd per block and queue.  Every thread of the block calls
+// it together.  The stage kernels push an entry or two per ray into two or
+// three queues, and the additions to one counter complete one after the other
+// (about 1.3 per ns on a B200): one per warp kept a shading stage at 0.2 ms
+// per 4M rays whatever else it did.
+template <int QUEUES, int WARPS>
+struct BlockClaim {
+    uint32_t count[QUEUES][WARPS];  // per warp, then each warp's first slot
+    __device__ __forceinline__ void operator()(const bool (&want)[QUEUES], uint32_t* const (&counter)[QUEUES],
+                                               uint32_t (&slot)[QUEUES]) {
+        static_assert(QUEUES <= WARPS, "warp k adds up queue k");
+        const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
+        unsigned mask[QUEUES];
+#pragma unroll
+        for (int k = 0; k < QUEUES; ++k) {
+            mask[k] = __ballot_sync(0xffffffffu, want[k]);
+            if (lane == 0) count[k][wid] = (uint32_t)__popc(mask[k]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < QUEUES; ++k) {
+            if ((int)wid != k) continue;
+            const uint32_t n = lane < WARPS ? count[k][lane] : 0u;
+            uint32_t before = n;  // inclusive prefix over the warps
+#pragma unroll
+            for (int o = 1; o < WARPS; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, before, o);
+                if ((int)lane >= o) before += v;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, before, WARPS - 1);
+            uint32_t base = 0;
+            if (lane == 0 && total) base = atomicAdd(counter[k], total);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (lane < WARPS) count[k][lane] = base + before - n;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < QUEUES; ++k) slot[k] = count[k][wid] + (uint32_t)__popc(mask[k] & ((1u << lane) - 1u));
+    }
+};
+
 constexpr int TRACE_NODE_STEPS = 3;
 constexpr int TRACE_REFILL = 12;
 
