@@ -604,47 +604,126 @@ __global__ void k_gdpt_init(uint32_t w, uint32_t h, float* __restrict__ recon, c
     }
 }
 
-__device__ __forceinline__ float median4(float v0, float v1, float v2, float v3) {  // compute_median :275-301
-    const float v[4] = {v0, v1, v2, v3};
-    float med = 0.0f;
-    uint32_t amin = 0, amax = 0;
-#pragma unroll
-    for (uint32_t i = 0; i < 4; ++i) {
-        med += v[i];
-        if (v[i] < v[amin]) amin = i;
-        if (v[i] > v[amax]) amax = i;
-    }
-    return (med - v[amin] - v[amax]) / 2.0f;
+// compute_median (:275-301): the mean of the two middle values, the sum taken
+// in the arguments' order.
+__device__ __forceinline__ float median4(float v0, float v1, float v2, float v3) {
+    const float lo = fminf(min3(v0, v1, v2), v3), hi = fmaxf(max3(v0, v1, v2), v3);
+    return (v0 + v1 + v2 + v3 - lo - hi) / 2.0f;
 }
 
-// optimization_kernel (GradientDomain.cu:303-350): src -> dst (interior).
-// copy_border: the border pixels of dst take src's (see
-// launch_gdpt_reconstruct).  Launched as a chain of programmatic dependent
-// launches: each pass lets the next one be scheduled as soon as its own
-// blocks start, and waits for the previous pass to complete (and its
-// writes to be visible) before it reads anything, so the 50 short passes
-// overlap their launch latencies instead of paying them one after another.
-__global__ void k_gdpt_opt(uint32_t w, uint32_t h, const float* __restrict__ src, const float* __restrict__ gx,
-                           const float* __restrict__ gy, float* __restrict__ dst, int copy_border) {
+// GD_PASSES passes of optimization_kernel (GradientDomain.cu:303-350), the
+// passes first, first + 1, .. of the reconstruction, src -> dst.  A block
+// holds a region of GD_COLS x (GD_SEGS * GD_ROWS) pixels, GD_PASSES more on
+// every side than the tile it writes: each pass leaves one more ring of
+// the region undefined.  A thread keeps GD_ROWS values of one float column
+// (column and channel: columns 3 floats apart are neighbours) and their
+// gradients in registers for all passes and reads only its left and right
+// neighbours, and the rows next to its own, from shared memory.
+// Border pixels of the image are no pass's output.  The reference copies the
+// whole of temp, its border included, over the output after every pass
+// (:392-401): pass 0 reads the border that k_gdpt_init gave the output, every
+// later one temp's, and the output's border ends as temp's (copy_border).
+//
+// One pass per launch pays a launch's latency for 0.5 us of arithmetic at
+// 512 x 512 (and re-reads 48 B per pixel through L2 at larger sizes); here a
+// region is read once for five.  Bound by issue (17 instructions a value and
+// pass, 1.7 times the values for the rings) and, below 512 x 512, by a block's
+// latency.  Reconstruction on a B200, one pass per launch -> this: 64 x 48 149
+// -> 118 us, 512 x 512 217 -> 132 (137 tiles on 148 SMs), 1280 x 720 535 -> 365,
+// 1920 x 1080 1300 -> 750; 3 segments of 16 rows 169 at 512 x 512, 5 of 10 143.
+// Launched as a chain of programmatic dependent launches: each
+// lets the next be scheduled when its own blocks start, which waits for it
+// to complete before it reads anything.
+constexpr int GD_PASSES = 5, GD_COLS = 64, GD_SEGS = 4, GD_ROWS = 12;
+constexpr int GD_TILE_W = GD_COLS - 2 * GD_PASSES, GD_TILE_H = GD_SEGS * GD_ROWS - 2 * GD_PASSES;
+constexpr int GD_ROW_FLOATS = 3 * GD_COLS, GD_THREADS = GD_ROW_FLOATS * GD_SEGS;
+constexpr int GD_PLANE = GD_SEGS * GD_ROWS * GD_ROW_FLOATS;  // floats of a region
+constexpr int GD_PAD = GD_ROW_FLOATS;                        // a row before and after it
+constexpr size_t GD_SMEM = sizeof(float) * 2 * (GD_PLANE + 2 * GD_PAD);
+
+// EDGE: the region reaches the image's border or beyond.
+template <bool EDGE>
+__device__ __forceinline__ void gdpt_region(uint32_t w, uint32_t h, const float* src, const float* __restrict__ gx,
+                                            const float* __restrict__ gy, const float* temp, float* dst, int first,
+                                            int copy_border, float* cur, float* nxt) {
+    const int col = (int)(threadIdx.x % GD_ROW_FLOATS), row0 = (int)(threadIdx.x / GD_ROW_FLOATS) * GD_ROWS;
+    const int x = (int)blockIdx.x * GD_TILE_W - GD_PASSES + col / 3, c = col % 3;
+    const int y0 = (int)blockIdx.y * GD_TILE_H - GD_PASSES + row0;
+    const int W = (int)w, H = (int)h;
+    const bool in_x = !EDGE || (x >= 0 && x < W);
+    const ptrdiff_t pitch = 3 * (ptrdiff_t)w, at0 = (ptrdiff_t)y0 * pitch + 3 * (ptrdiff_t)x + c;
+    float v[GD_ROWS], gxl[GD_ROWS], gxp[GD_ROWS], gyp[GD_ROWS];
+    float gyd = 0.0f;    // gy one row below the thread's first
+    uint32_t inner = 0;  // EDGE: rows whose pixel a pass computes
+#pragma unroll
+    for (int r = 0; r < GD_ROWS; ++r) {
+        const int y = y0 + r;
+        const ptrdiff_t p = at0 + r * pitch;
+        if (!EDGE) {
+            v[r] = src[p];
+            gxp[r] = __ldg(&gx[p]);
+            gxl[r] = __ldg(&gx[p - 3]);
+            gyp[r] = __ldg(&gy[p]);
+        } else {
+            v[r] = gxl[r] = gxp[r] = gyp[r] = 0.0f;
+            if (in_x && y >= 0 && y < H) {
+                v[r] = src[p];
+                if (x > 0 && y > 0 && x < W - 1 && y < H - 1) {
+                    inner |= 1u << r;
+                    gxp[r] = __ldg(&gx[p]);
+                    gxl[r] = __ldg(&gx[p - 3]);
+                }
+                gyp[r] = __ldg(&gy[p]);
+            }
+        }
+    }
+    if (!EDGE || (in_x && y0 > 0 && y0 <= H)) gyd = __ldg(&gy[at0 - pitch]);
+#pragma unroll
+    for (int r = 0; r < GD_ROWS; ++r) cur[(row0 + r) * GD_ROW_FLOATS + col] = v[r];
+    __syncthreads();
+    for (int p = 0; p < GD_PASSES; ++p) {
+        float below = cur[(row0 - 1) * GD_ROW_FLOATS + col], gb = gyd;
+        const float above = cur[(row0 + GD_ROWS) * GD_ROW_FLOATS + col];
+#pragma unroll
+        for (int r = 0; r < GD_ROWS; ++r) {
+            const float* q = cur + (row0 + r) * GD_ROW_FLOATS + col;
+            const float old = v[r];
+            const float m = median4(q[-3] + gxl[r], below + gb, q[3] - gxp[r],
+                                    (r + 1 < GD_ROWS ? v[r + 1] : above) - gyp[r]);
+            below = old;
+            gb = gyp[r];
+            if (!EDGE || (inner >> r & 1u)) v[r] = m;
+            else if (first + p == 0 && in_x && y0 + r >= 0 && y0 + r < H) v[r] = temp[at0 + r * pitch];
+            nxt[(row0 + r) * GD_ROW_FLOATS + col] = v[r];
+        }
+        float* t = cur;
+        cur = nxt;
+        nxt = t;
+        __syncthreads();
+    }
+    if (!in_x || col < 3 * GD_PASSES || col >= 3 * (GD_COLS - GD_PASSES)) return;
+#pragma unroll
+    for (int r = 0; r < GD_ROWS; ++r) {
+        const int y = y0 + r, row = row0 + r;
+        if (row < GD_PASSES || row >= GD_SEGS * GD_ROWS - GD_PASSES) continue;
+        if (!EDGE || (y >= 0 && y < H && ((inner >> r & 1u) || copy_border))) dst[at0 + r * pitch] = v[r];
+    }
+}
+
+__global__ void __launch_bounds__(GD_THREADS, 1) k_gdpt_opt(uint32_t w, uint32_t h, const float* src,
+                                                            const float* __restrict__ gx,
+                                                            const float* __restrict__ gy, const float* temp, float* dst,
+                                                            int first, int copy_border) {
+    extern __shared__ float s_gd[];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (tid >= w * h) return;
-    const uint32_t y = tid / w, x = tid - w * y;
-    if (x == 0 || y == 0 || x == w - 1 || y == h - 1) {
-        if (copy_border)
-            for (int c = 0; c < 3; ++c) dst[3 * (size_t)tid + c] = src[3 * (size_t)tid + c];
-        return;
-    }
-    const size_t p = tid, l = p - 1, r = p + 1, u = p + w, dn = p - w;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const float v1 = src[3 * l + c] + gx[3 * l + c];
-        const float v2 = src[3 * dn + c] + gy[3 * dn + c];
-        const float v3 = src[3 * r + c] - gx[3 * p + c];
-        const float v4 = src[3 * u + c] - gy[3 * p + c];
-        dst[3 * p + c] = median4(v1, v2, v3, v4);
-    }
+    float* cur = s_gd + GD_PAD;
+    float* nxt = cur + GD_PLANE + 2 * GD_PAD;
+    // the region's pixels and one more below and left of it lie inside the border
+    const int x0 = (int)blockIdx.x * GD_TILE_W - GD_PASSES, y0 = (int)blockIdx.y * GD_TILE_H - GD_PASSES;
+    const bool inside = x0 > 1 && y0 > 1 && x0 + GD_COLS < (int)w && y0 + GD_SEGS * GD_ROWS < (int)h;
+    if (inside) gdpt_region<false>(w, h, src, gx, gy, temp, dst, first, copy_border, cur, nxt);
+    else gdpt_region<true>(w, h, src, gx, gy, temp, dst, first, copy_border, cur, nxt);
 }
 
 // raytracing_kernel (RayTracer.cu:11-54): direct light from every light's
@@ -702,28 +781,29 @@ cudaError_t launch_gdpt_reconstruct(uint32_t w, uint32_t h, const float* base, c
     const uint32_t n = w * h;
     if (n == 0) return cudaSuccess;
     k_gdpt_init<<<(n + 255) / 256, 256, 0, st>>>(w, h, out, base, gxf, gxb, gyf, gyb, gx, gy);
-    // GradientDomain.cu:392-401: 50 passes, each followed by a copy of the
-    // whole of temp (its border included, which no pass writes) into the
-    // output.  Here the passes alternate between the output and temp instead:
-    // pass 0 reads the output with the border k_gdpt_init gave it; every
-    // later pass must see temp's border there, so the passes that write the
-    // output also copy temp's border into it.  The result lands in the output
-    // after the even number of passes, as the reference's does.
+    // 50 passes (GradientDomain.cu:392-401), alternating between the output and
+    // temp instead of copying temp back after each: the result lands in the
+    // output after an even number of launches.
+    constexpr int LAUNCHES = 50 / GD_PASSES;
+    static_assert(LAUNCHES * GD_PASSES == 50 && LAUNCHES % 2 == 0, "passes per launch");
+    static const cudaError_t smem =
+        cudaFuncSetAttribute(k_gdpt_opt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GD_SMEM);
+    if (smem != cudaSuccess) return smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((n + 255) / 256);
-    cfg.blockDim = dim3(256);
+    cfg.gridDim = dim3((w + GD_TILE_W - 1) / GD_TILE_W, (h + GD_TILE_H - 1) / GD_TILE_H);
+    cfg.blockDim = dim3(GD_THREADS);
+    cfg.dynamicSmemBytes = GD_SMEM;
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    for (int i = 0; i < 50; ++i) {
+    for (int i = 0; i < LAUNCHES; ++i) {
         const float* src = (i & 1) ? temp : out;
         float* dst = (i & 1) ? out : temp;
-        const float* cgx = gx;
-        const float* cgy = gy;
-        cudaError_t e = cudaLaunchKernelEx(&cfg, k_gdpt_opt, w, h, src, cgx, cgy, dst, i & 1);
+        const float *cgx = gx, *cgy = gy, *ctemp = temp;
+        cudaError_t e = cudaLaunchKernelEx(&cfg, k_gdpt_opt, w, h, src, cgx, cgy, ctemp, dst, i * GD_PASSES, i & 1);
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
