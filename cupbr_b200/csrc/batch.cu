@@ -327,113 +327,110 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch_persistent(con
     if (overflow) atomicAdd(err, 1u);
 }
 
-// Adjoint of the persistent kernel's frames with respect to the scenes'
-// albedo textures (batch_launch_backward): each thread replays its path of
-// every frame from the path's seed -- the same camera ray, traversal and
-// shading, so the same vertices -- and records, at each textured Lambert
-// vertex, the texel and the radiance gathered before that vertex's light
-// term.  Every radiance term from that light term on carries the texel's
-// albedo exactly once per channel (Lambert sampling does not depend on the
-// albedo; Russian roulette is off), so its derivative with respect to the
-// texel is (path radiance - radiance before) / albedo, scattered with
-// weight dLoss/dImage / (frame0 + spp) (the running mean's weight of one
-// frame).
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch_backward(const DeviceScene* __restrict__ scenes,
-                                                            const BatchView* __restrict__ views,
-                                                            const BatchItem* __restrict__ items, uint32_t n_items,
-                                                            uint32_t* counter, uint32_t max_depth,
-                                                            const float* const* __restrict__ grad_img,
-                                                            float* const* __restrict__ grad_tex, uint32_t* err) {
-    constexpr int WARPS = THREADS / 32;
-    constexpr int WORDS = (int)(sizeof(DeviceScene) / sizeof(uint32_t));
-    __shared__ DeviceScene s_scene[WARPS];
-    const unsigned full = 0xffffffffu;
-    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-    DeviceScene& S = s_scene[wid];
-    uint32_t cur_scene = 0xFFFFFFFFu;
-    bool overflow = false;
-    TraceCounters tc;
-    PTFrame F{};
-    F.max_depth = max_depth;
-    F.use_rr = 0;
-    const CacheFrame C{};
-    for (;;) {
-        uint32_t it = 0;
-        if (lane == 0) it = atomicAdd(counter, 1u);
-        it = __shfl_sync(full, it, 0);
-        if (it >= n_items) break;
-        const BatchItem bi = items[it];
-        const BatchView v = views[bi.view];
-        if (v.scene != cur_scene) {
-            __syncwarp();
-            const uint32_t* src = reinterpret_cast<const uint32_t*>(scenes + v.scene);
-            uint32_t* dst = reinterpret_cast<uint32_t*>(&S);
-            for (int k = (int)lane; k < WORDS; k += 32) dst[k] = __ldg(&src[k]);
-            __syncwarp();
-            cur_scene = v.scene;
-        }
-        float* gt = grad_tex[v.scene];
-        const float* gi = grad_img[bi.view];
-        const uint32_t pixels = v.width * v.height;
-        const uint32_t slot = bi.slot0 + lane;
-        if (!gt || !gi || !S.tex || slot >= pixels) continue;
-        const uint32_t tid = slot_pixel(slot, v.width, v.height);
-        const float inv_n = 1.0f / ((float)v.frame0 + (float)v.spp);
-        const f3 g = mk(gi[3 * (size_t)tid], gi[3 * (size_t)tid + 1], gi[3 * (size_t)tid + 2]) * inv_n;
-        if (g.x == 0.0f && g.y == 0.0f && g.z == 0.0f) continue;
-        const uint32_t py = tid / v.width, px = tid - v.width * py;
-        for (uint32_t fr = 0; fr < v.spp; ++fr) {
-            const uint32_t f = v.frame0 + fr;
-            uint32_t seed = tea4(tid, f);
+// ---- texture adjoint (batch_launch_backward) ----------------------------
+// The frames of a launch replayed from the paths' seeds as wavefronts: the
+// same camera rays, traversal and shading, so the same vertices.  The shading
+// stage records, at each textured Lambert vertex, the texel and the radiance
+// gathered before that vertex's light term (TexRecord).  Every radiance term
+// from that light term on carries the texel's albedo exactly once per channel
+// (Lambert sampling does not depend on the albedo; Russian roulette is off),
+// so its derivative with respect to the texel is (path radiance - radiance
+// before) / albedo, scattered once the wavefront is done with weight
+// dLoss/dImage / (frame0 + spp) (the running mean's weight of one frame).
+// One thread per path through all of its bounces (128 registers, 16 warps per
+// SM, every bounce as long as its slowest path) took 10.7 ms for 12 views of
+// three textured scenes (256 x 256 x 16, depth 5) on a B200; this 4.3.
+
+// Path q of a scene (its views' frames one after the other): view, pixel,
+// frame, and the pixel's weight (0 for a view without an image gradient).
+__device__ __forceinline__ f3 backward_path(const BatchBackwardSegment* __restrict__ segs, uint32_t nseg,
+                                            const BatchView* __restrict__ views,
+                                            const float* const* __restrict__ grad_img, uint64_t q, uint32_t& view,
+                                            uint32_t& tid, uint32_t& frame) {
+    uint32_t lo = 0, hi = nseg;
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (segs[mid].start <= q) lo = mid;
+        else hi = mid;
+    }
+    view = segs[lo].view;
+    const BatchView& v = views[view];
+    const uint32_t pixels = v.width * v.height;
+    const uint64_t local = q - segs[lo].start;
+    const uint32_t fr = (uint32_t)(local / pixels);
+    tid = slot_pixel((uint32_t)(local - (uint64_t)fr * pixels), v.width, v.height);
+    frame = v.frame0 + fr;
+    const float* gi = grad_img[view];
+    if (!gi) return splat(0.0f);
+    const float inv_n = 1.0f / ((float)v.frame0 + (float)v.spp);
+    return mk(gi[3 * (size_t)tid], gi[3 * (size_t)tid + 1], gi[3 * (size_t)tid + 2]) * inv_n;
+}
+
+// Camera rays (batch_camera_slot) of the wavefront's paths p0 .. p0 + n - 1 of
+// its scene; those of weight 0 are not traced.
+__global__ void __launch_bounds__(256) k_backward_camera(const BatchBackwardSegment* __restrict__ segs, uint32_t nseg,
+                                                         const BatchView* __restrict__ views,
+                                                         const float* const* __restrict__ grad_img, Workspace W,
+                                                         TexRecord R, uint64_t p0, uint32_t n) {
+    __shared__ BlockClaim<1, 8> s_claim;
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    bool want = false;
+    float4 q0, q1;
+    if (i < n) {
+        uint32_t view, tid, frame;
+        want = !is_zero(backward_path(segs, nseg, views, grad_img, p0 + i, view, tid, frame));
+        R.depths[i] = 0u;
+        W.radiance[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (want) {
+            const BatchView& v = views[view];
+            uint32_t seed = tea4(tid, frame);
+            const uint32_t py = tid / v.width, px = tid - v.width * py;
             const float jx = rnd(seed);
             const float jy = rnd(seed);
             const float rx = 2.0f * (((float)px + jx) / (float)v.width - 0.5f);
             const float ry = 2.0f * (((float)py + jy) / (float)v.height - 0.5f);
             const f3 wp = v.cam_pos + v.cam_z + rx * v.cam_x + ry * v.cam_y;
-            float4 q0 = f4(v.cam_pos, __uint_as_float(tid));
-            float4 q1 = f4(normalize(wp - v.cam_pos), __uint_as_float(seed));
-            float4 q2 = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-            f3 rad = splat(0.0f);
-            int32_t rec_t[BATCH_BWD_MAX_DEPTH];
-            f3 rec_c[BATCH_BWD_MAX_DEPTH];
-            uint32_t nrec = 0;
-            for (uint32_t d = 0;; ++d) {
-                float t;
-                int32_t prim;
-                uint32_t key;
-                trace_scene_rt(false, false, S, xyz(q0), xyz(q1), 0.0f, t, prim, key, overflow, tc);
-                ShadeOut so;
-                shade_core<false, false>(S, F, C, d, q0, q1, q2, make_float2(t, __int_as_float(prim)), rad, so);
-                if (so.texel >= 0 && nrec < BATCH_BWD_MAX_DEPTH) {
-                    rec_t[nrec] = so.texel;
-                    rec_c[nrec] = rad;
-                    ++nrec;
-                }
-                if (so.sh) {
-                    float ts;
-                    int32_t ps;
-                    uint32_t ks;
-                    if (!trace_scene_rt(true, false, S, xyz(so.s0), xyz(so.s1), so.s0.w, ts, ps, ks,
-                                        overflow, tc))
-                        rad += xyz(so.s2);
-                }
-                if (!so.ext) break;
-                q0 = so.e0;
-                q1 = so.e1;
-                q2 = so.e2;
-            }
-            for (uint32_t k = 0; k < nrec; ++k) {
-                const f3 a = xyz(S.tex[rec_t[k]]);
-                const f3 after = rad - rec_c[k];
-                float* o = gt + 3 * (size_t)rec_t[k];
-                if (a.x > 0.0f && after.x != 0.0f) atomicAdd(o, g.x * after.x / a.x);
-                if (a.y > 0.0f && after.y != 0.0f) atomicAdd(o + 1, g.y * after.y / a.y);
-                if (a.z > 0.0f && after.z != 0.0f) atomicAdd(o + 2, g.z * after.z / a.z);
-            }
+            q0 = f4(v.cam_pos, __uint_as_float(i));
+            q1 = f4(normalize(wp - v.cam_pos), __uint_as_float(seed));
         }
     }
-    if (overflow) atomicAdd(err, 1u);
+    uint32_t slot[1];
+    s_claim({want}, {&W.ctr[CTR_RAYS + 0]}, slot);
+    if (!want) return;
+    float4* q = W.rays[0] + 3 * (size_t)slot[0];
+    q[0] = q0;
+    q[1] = q1;
+    q[2] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+}
+
+__global__ void __launch_bounds__(256, 4) k_backward_shade(DeviceScene S, PTFrame F, Workspace W, uint32_t depth,
+                                                           TexRecord R) {
+    shade_stage<false, false, true, true>(S, F, W, depth, CacheFrame{}, R);
+}
+
+// The recorded vertices of the wavefront's paths into the texture's gradient.
+__global__ void __launch_bounds__(256) k_backward_scatter(const BatchBackwardSegment* __restrict__ segs, uint32_t nseg,
+                                                          const BatchView* __restrict__ views,
+                                                          const float* const* __restrict__ grad_img, Workspace W,
+                                                          TexRecord R, const float4* __restrict__ tex,
+                                                          float* __restrict__ grad_tex, uint64_t p0, uint32_t n) {
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= n) return;
+    uint32_t depths = R.depths[i];
+    if (!depths) return;
+    uint32_t view, tid, frame;
+    const f3 g = backward_path(segs, nseg, views, grad_img, p0 + i, view, tid, frame);
+    const f3 rad = xyz(W.radiance[i]);
+    for (; depths; depths &= depths - 1u) {
+        const float4 r = R.vertex[(size_t)(__ffs((int)depths) - 1) * R.stride + i];
+        const int32_t texel = __float_as_int(r.w);
+        const f3 a = xyz(__ldg(&tex[texel]));
+        const f3 after = rad - xyz(r);
+        float* o = grad_tex + 3 * (size_t)texel;
+        if (a.x > 0.0f && after.x != 0.0f) atomicAdd(o, g.x * after.x / a.x);
+        if (a.y > 0.0f && after.y != 0.0f) atomicAdd(o + 1, g.y * after.y / a.y);
+        if (a.z > 0.0f && after.z != 0.0f) atomicAdd(o + 2, g.z * after.z / a.z);
+    }
 }
 
 }  // namespace
@@ -496,32 +493,29 @@ cudaError_t batch_launch_coop(const DeviceScene* scenes, const BatchWave* waves,
     return cudaLaunchKernelEx(&cfg, k_batch_coop, scenes, waves, n_waves, segs, views, w, max_depth, gb, probe_ns);
 }
 
-cudaError_t batch_launch_backward(const DeviceScene* scenes, const BatchView* views, const BatchItem* items,
-                                  uint32_t n_items, uint32_t* counter, uint32_t max_depth, const float* const* grad_img,
-                                  float* const* grad_tex, uint32_t threads, uint32_t blocks_per_sm, int num_sms,
-                                  uint32_t* err, cudaStream_t st) {
+cudaError_t batch_launch_backward(const DeviceScene& S, const BatchBackwardSegment* segs, uint32_t nseg,
+                                  const BatchView* views, uint64_t paths, const Workspace& W, const TexRecord& R,
+                                  uint32_t max_depth, const float* const* grad_img, float* grad_tex, int num_sms,
+                                  cudaStream_t st) {
     if (max_depth > BATCH_BWD_MAX_DEPTH) return cudaErrorInvalidValue;
-    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), st);
-    if (e != cudaSuccess) return e;
-    const uint32_t blocks = std::max(1u, blocks_per_sm) * (uint32_t)num_sms;
-    if (threads == 64)
-        k_batch_backward<64><<<blocks, 64, 0, st>>>(scenes, views, items, n_items, counter, max_depth, grad_img,
-                                                    grad_tex, err);
-    else if (threads == 256)
-        k_batch_backward<256><<<blocks, 256, 0, st>>>(scenes, views, items, n_items, counter, max_depth, grad_img,
-                                                      grad_tex, err);
-    else
-        k_batch_backward<128><<<blocks, 128, 0, st>>>(scenes, views, items, n_items, counter, max_depth, grad_img,
-                                                      grad_tex, err);
-    return cudaGetLastError();
-}
-
-int batch_backward_occupancy(uint32_t threads) {
-    int b = 0;
-    if (threads == 64) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_batch_backward<64>, 64, 0);
-    else if (threads == 256) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_batch_backward<256>, 256, 0);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_batch_backward<128>, 128, 0);
-    return b > 0 ? b : 1;
+    PTFrame F{};
+    F.max_depth = max_depth;
+    F.use_rr = 0;
+    for (uint64_t p0 = 0; p0 < paths; p0 += R.stride) {
+        const uint32_t n = (uint32_t)std::min<uint64_t>(R.stride, paths - p0);
+        cudaError_t e = cudaMemsetAsync(W.ctr, 0, sizeof(uint32_t) * CTR_TOTAL, st);
+        if (e != cudaSuccess) return e;
+        k_backward_camera<<<(n + 255) / 256, 256, 0, st>>>(segs, nseg, views, grad_img, W, R, p0, n);
+        for (uint32_t d = 0; d < max_depth; ++d) {
+            e = d == 0 ? pt_launch_extend_camera(S, W, num_sms, st) : pt_launch_extend(S, W, d, num_sms, st);
+            if (e != cudaSuccess) return e;
+            k_backward_shade<<<num_sms * 8, 256, 0, st>>>(S, F, W, d, R);
+            if ((e = pt_launch_connect(S, W, d, num_sms, st)) != cudaSuccess) return e;
+        }
+        k_backward_scatter<<<(n + 255) / 256, 256, 0, st>>>(segs, nseg, views, grad_img, W, R, S.tex, grad_tex, p0, n);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 template <bool PACKET>

@@ -97,18 +97,31 @@ int batch_persistent_occupancy(uint32_t threads, bool packet);
 
 // Deepest path the albedo-texture adjoint records (vertices per path).
 constexpr uint32_t BATCH_BWD_MAX_DEPTH = 16;
-// Adjoint of the persistent kernel's frames with respect to the scenes'
-// albedo textures: grad_tex[scene] (tex_w * tex_h RGB floats, or null) +=
-// the derivative of sum over views and pixels of grad_img[view][pixel] .
-// image[pixel] (grad_img[view] width * height RGB floats, or null), each
-// view's image taken as the mean of its frames 0 .. frame0 + spp - 1 and
-// only the frames frame0 .. frame0 + spp - 1 replayed (exact when frame0 = 0).
-// max_depth <= BATCH_BWD_MAX_DEPTH.  Same work items and counter protocol
-// as the forward kernel.
-cudaError_t batch_launch_backward(const DeviceScene* scenes, const BatchView* views, const BatchItem* items,
-                                  uint32_t n_items, uint32_t* counter, uint32_t max_depth, const float* const* grad_img,
-                                  float* const* grad_tex, uint32_t threads, uint32_t blocks_per_sm, int num_sms,
-                                  uint32_t* err, cudaStream_t st);
-int batch_backward_occupancy(uint32_t threads);
+// Consecutive paths of one scene in the adjoint's order: view by view, frame by
+// frame; `start` is the view's first.
+struct BatchBackwardSegment {
+    uint64_t start;
+    uint32_t view, pad;
+};
+// What the texture adjoint keeps of a wavefront: per path a mask of the depths
+// with a textured Lambert vertex, and per depth and path that vertex's texel
+// and the radiance gathered before its light term.
+struct TexRecord {
+    float4* vertex;    // depth * stride + path: (radiance, texel)
+    uint32_t* depths;  // per path
+    uint32_t stride;   // paths of a wavefront
+};
+// Adjoint of a launch's frames with respect to the albedo texture of scene S:
+// grad_tex (tex_w * tex_h RGB floats) += the derivative of the sum over the
+// scene's views and pixels of grad_img[view][pixel] . image[pixel]
+// (grad_img[view] width * height RGB floats, or null), each view's image taken
+// as the mean of its frames 0 .. frame0 + spp - 1 and only the frames frame0 ..
+// frame0 + spp - 1 replayed (exact when frame0 = 0).  `paths` paths in
+// wavefronts of R.stride; W and R hold that many.  max_depth <=
+// BATCH_BWD_MAX_DEPTH.
+cudaError_t batch_launch_backward(const DeviceScene& S, const BatchBackwardSegment* segs, uint32_t nseg,
+                                  const BatchView* views, uint64_t paths, const Workspace& W, const TexRecord& R,
+                                  uint32_t max_depth, const float* const* grad_img, float* grad_tex, int num_sms,
+                                  cudaStream_t st);
 
 }  // namespace cupbr_b200

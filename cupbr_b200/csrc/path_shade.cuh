@@ -3,6 +3,7 @@
 // (batch.cu).
 #pragma once
 
+#include "batch.hpp"
 #include "cache.hpp"
 #include "pathtracer.hpp"
 #include "shading.cuh"
@@ -212,14 +213,18 @@ __device__ __forceinline__ uint32_t shade_class(const DeviceScene& S, float2 h) 
     return type == 4 ? 2u : (type == 2 || type == 3) ? 3u : 1u;
 }
 
-template <bool CACHE, bool PHYS, bool NC = true>
+template <bool CACHE, bool PHYS, bool NC = true, bool REC = false>
 __device__ __forceinline__ void shade_one(const DeviceScene& S, const PTFrame& F, const Workspace& W,
                                           const CacheFrame& C, uint32_t depth, const float4& q0, const float4& q1,
-                                          const float4& q2, float2 h, ShadeOut& so) {
+                                          const float4& q2, float2 h, ShadeOut& so, const TexRecord& R = TexRecord{}) {
     const uint32_t pid = __float_as_uint(q0.w);
     f3 rad = xyz(NC ? W.radiance[pid] : __ldcg(&W.radiance[pid]));
     shade_core<CACHE, PHYS>(S, F, C, depth, q0, q1, q2, h, rad, so);
     W.radiance[pid] = f4(rad, 0.0f);
+    if (REC && so.texel >= 0) {
+        R.vertex[(size_t)depth * R.stride + pid] = f4(rad, __int_as_float(so.texel));
+        R.depths[pid] |= 1u << depth;
+    }
 }
 
 // The shading stage of one depth over ray queue[depth] with blocks of 256
@@ -227,9 +232,9 @@ __device__ __forceinline__ void shade_one(const DeviceScene& S, const PTFrame& F
 // kernel's shading stage): each chunk is shaded in material-class order
 // (misses, diffuse, GGX, delta), so most warps run one BSDF.  A queue below
 // C.tail_threshold is left to k_tail.
-template <bool CACHE, bool PHYS, bool NC = true>
+template <bool CACHE, bool PHYS, bool NC = true, bool REC = false>
 __device__ __forceinline__ void shade_stage(const DeviceScene& S, const PTFrame& F, const Workspace& W, uint32_t depth,
-                                            const CacheFrame& C) {
+                                            const CacheFrame& C, const TexRecord& R = TexRecord{}) {
     const uint32_t count = NC ? W.ctr[CTR_RAYS + depth] : __ldcg(&W.ctr[CTR_RAYS + depth]);
     if (count < C.tail_threshold) return;
     const float4* __restrict__ q = W.rays[depth & 1];
@@ -275,7 +280,7 @@ __device__ __forceinline__ void shade_stage(const DeviceScene& S, const PTFrame&
             const float4 q0 = qload<NC>(&q[3 * (size_t)i]);
             const float4 q1 = qload<NC>(&q[3 * (size_t)i + 1]);
             const float4 q2 = qload<NC>(&q[3 * (size_t)i + 2]);
-            shade_one<CACHE, PHYS, NC>(S, F, W, C, depth, q0, q1, q2, NC ? W.hits[i] : __ldcg(&W.hits[i]), so);
+            shade_one<CACHE, PHYS, NC, REC>(S, F, W, C, depth, q0, q1, q2, NC ? W.hits[i] : __ldcg(&W.hits[i]), so, R);
         }
         uint32_t slot[QUEUES];
         if constexpr (CACHE) {
