@@ -242,12 +242,21 @@ struct cupbr_renderer_s {
     cudaStream_t stream = nullptr;
     uint64_t last_rays[2] = {0, 0};
     uint32_t batch_paths = 1u << 25;  // paths per wavefront when several frames are rendered at once
-    // per-path tail kernel below this queue size (0: off); unless set, 2^17
-    // on one stream and 2^16 pipelined, where the other stream's wavefront
-    // fills the SMs that a sparse queue leaves idle
+    // per-path tail kernel below this queue size (0: off); see tail()
     uint32_t tail_paths = 0;
     bool tail_set = false;
-    uint32_t tail() const { return tail_set ? tail_paths : (pipelined ? 0u : 1u << 17); }
+    // A frame of few paths does not fill the device: one launch for all of it
+    // beats the stage kernels up to 3 x 2^17 paths (Cornell box, spheres, terrain
+    // at 512 x 512: 334 against 402 us, 444 / 506, 875 / 1030; at 960 x 540
+    // 506 / 516, 606 / 589, 1357 / 1278; at 256 x 256 138 / 255, 196 / 374,
+    // 513 / 729; eight pipelined 256 x 256 frames 1117 / 2153, 1594 / 3397,
+    // 4149 / 8085).  The end of a larger frame pays below 2^15 rays (terrain
+    // 960 x 540 1277 against 1376 us), not pipelined, where the next frame's
+    // wavefront fills the SMs that a sparse queue leaves idle.
+    PTTail tail() const {
+        if (tail_set) return {tail_paths, tail_paths};
+        return {pipelined ? 0u : 1u << 15, 3u << 17};
+    }
     // rays of the last wavefront frame: closest-hit and shadow queue sizes
     cudaError_t read_wavefront_rays() {
         uint32_t c[CTR_TOTAL];

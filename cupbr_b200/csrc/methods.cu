@@ -629,7 +629,7 @@ __device__ __forceinline__ float median4(float v0, float v1, float v2, float v3)
 // region is read once for five.  Bound by issue (17 instructions a value and
 // pass, 1.7 times the values for the rings) and, below 512 x 512, by a block's
 // latency.  Reconstruction on a B200, one pass per launch -> this: 64 x 48 149
-// -> 118 us, 512 x 512 217 -> 132 (137 tiles on 148 SMs), 1280 x 720 535 -> 365,
+// -> 118 us, 512 x 512 217 -> 132 (140 tiles on 148 SMs), 1280 x 720 535 -> 365,
 // 1920 x 1080 1300 -> 750; 3 segments of 16 rows 169 at 512 x 512, 5 of 10 143.
 // Launched as a chain of programmatic dependent launches: each
 // lets the next be scheduled when its own blocks start, which waits for it

@@ -20,7 +20,8 @@ constexpr uint32_t CTR_TFETCH = 256;  // [d]: work-fetch cursor of the medium's 
 constexpr uint32_t CTR_FFETCH = 320;  // [d]: work-fetch cursor of the medium's free-flight kernel
 constexpr uint32_t CTR_MVERT = 384;   // [d]: medium vertices of depth d
 constexpr uint32_t CTR_SVERT = 448;   // [d]: surface vertices of depth d
-constexpr uint32_t CTR_TOTAL = 512;
+constexpr uint32_t CTR_RFETCH = 512;  // [d]: work-fetch cursor of the medium's light-term replay
+constexpr uint32_t CTR_TOTAL = 576;
 
 constexpr uint32_t ERR_STACK = 0;     // traversal stack overflows (entries dropped)
 constexpr uint32_t ERR_TOTAL = 8;
@@ -85,11 +86,16 @@ cudaError_t launch_trace_rays(const DeviceScene& S, uint32_t n, const float* o, 
 // k_connect, [last] after k_accumulate.
 // img == nullptr: the frame is traced but not accumulated (pt_launch_accumulate
 // does that, possibly on another stream).
-// tail_paths > 0: once a depth's ray queue holds fewer rays, one thread per
-// ray traces the rest of its path in one launch (same results; counted in
-// the closest-hit stage's events; never on count_stats frames).
+// tail (never on count_stats frames; same results; counted in the closest-hit
+// stage's events): once a depth's ray queue holds fewer than `paths` rays, one
+// thread per ray traces the rest of its path in one launch; a frame of fewer
+// than `whole_paths` paths goes to that launch whole and the stage kernels are
+// not launched.
+struct PTTail {
+    uint32_t paths = 0, whole_paths = 0;
+};
 cudaError_t pt_render_frame(const DeviceScene& S, const PTFrame& F, const Workspace& W, float* img, cudaStream_t st,
-                            int num_sms, bool count_stats, cudaEvent_t* ev = nullptr, uint32_t tail_paths = 0);
+                            int num_sms, bool count_stats, cudaEvent_t* ev = nullptr, PTTail tail = {});
 inline uint32_t pt_event_count(uint32_t max_depth) { return 3 + 3 * max_depth; }
 
 }  // namespace cupbr_b200
