@@ -33,7 +33,7 @@
 // vertices' light terms and next rays); k_medium_transmit (the light terms'
 // ratio tracking, persistent); then the shadow rays -- the path tracer's
 // k_connect when rendering the image, k_medium_connect in the gradient's two
-// replays.
+// replays, and k_medium_replay for the adjoint of the visible light terms.
 //
 // Adjoint (path replay, no stored vertices): a forward wavefront gives every
 // path's radiance L (summed in double); a second wavefront replays the same
@@ -121,34 +121,17 @@ __device__ __forceinline__ float dot3(f3 a, f3 b) { return a.x * b.x + a.y * b.y
 // the next direction), so it can run in a kernel of its own.
 __host__ __device__ __forceinline__ uint32_t ratio_seed(uint32_t path_seed) { return tea4(path_seed, 1u); }
 
-// Ratio-tracking transmittance of [0, len] along (o, d).  With g_grid the
-// walk adds scale * dlogT/dsigma_v = -scale / (sigma_bar - sigma_v) per point.
-__device__ __forceinline__ float ratio_track(const MediumGrid& G, f3 o, f3 d, float len, uint32_t& seed,
-                                             float* g_grid, float scale, bool& ovf, uint32_t& lookups) {
-    float ta, tb;
-    if (!box_interval(G, o, d, ta, tb)) return 1.0f;
-    tb = fminf(tb, len);
-    float T = 1.0f, t = ta;
-    for (int k = 0;; ++k) {
-        if (k == MEDIUM_MAX_EVENTS) {
-            ovf = true;
-            break;
-        }
-        t += free_step(G, seed);
-        if (!(t < tb)) break;
-        const uint32_t v = voxel_of(G, o + t * d);
-        const float s = __ldg(&G.density[v]);
-        ++lookups;
-        T *= 1.0f - s * G.inv_majorant;
-        if (g_grid) atomicAdd(&g_grid[v], -scale / (G.majorant - s));
-    }
-    return T;
+__device__ __forceinline__ f3 albedo_grad(f3 delta, f3 v, f3 albedo) {
+    return mk(albedo.x != 0.0f ? delta.x * v.x / albedo.x : 0.0f, albedo.y != 0.0f ? delta.y * v.y / albedo.y : 0.0f,
+              albedo.z != 0.0f ? delta.z * v.z / albedo.z : 0.0f);
 }
-
+__device__ __forceinline__ void add_params(float* g, f3 v) {
+    if (v.x != 0.0f) atomicAdd(&g[0], v.x);
+    if (v.y != 0.0f) atomicAdd(&g[1], v.y);
+    if (v.z != 0.0f) atomicAdd(&g[2], v.z);
+}
 __device__ __forceinline__ void add_albedo_grad(float* ga, f3 delta, f3 v, f3 albedo) {
-    if (albedo.x != 0.0f) atomicAdd(&ga[0], delta.x * v.x / albedo.x);
-    if (albedo.y != 0.0f) atomicAdd(&ga[1], delta.y * v.y / albedo.y);
-    if (albedo.z != 0.0f) atomicAdd(&ga[2], delta.z * v.z / albedo.z);
+    add_params(ga, albedo_grad(delta, v, albedo));
 }
 
 __device__ __forceinline__ f3 pixel_delta(const float* grad_img, uint32_t pixel, uint32_t spp) {
@@ -195,7 +178,12 @@ __global__ void k_medium_camera(MediumParams P, MediumBatch B, Workspace W, doub
     uint32_t seed = 0, p = 0;
     if (i < B.n_paths) {
         uint32_t fr, tid;
-        slot_path(i, P.width, P.height, B.frames, fr, tid);
+        if (MODE == ADJOINT) {  // frame by frame: the same pixel's paths at a time would add to the same voxels
+            fr = i / B.pixels;
+            tid = slot_pixel(i - fr * B.pixels, P.width, P.height);
+        } else {
+            slot_path(i, P.width, P.height, B.frames, fr, tid);
+        }
         p = fr * B.pixels + tid;
         seed = tea4(tid, B.sample0 + fr);
         const uint32_t py = tid / P.width, px = tid - P.width * py;
@@ -234,12 +222,19 @@ __global__ void k_medium_camera(MediumParams P, MediumBatch B, Workspace W, doub
 // hit, sorting the paths into medium vertices (a real collision; front of
 // `verts`) and surface vertices (back of `verts`): (position, path),
 // (direction, RNG state), (weight, primitive ref for a surface).
-// Persistent: a lane takes the next entry as soon as its flight ends (one
-// atomicAdd per warp) and advances in rounds of FLIGHT_ROUND steps, so
-// flights of different lengths keep a warp full.  The adjoint adds the
-// pending Lambert weight gradient of the previous vertex and the free-flight
-// gradients.
+// Persistent: lanes whose flights have ended hand in their vertices and take
+// the next entries (TraceShare) together, FLIGHT_REFILL of them or more, and
+// advance in rounds of FLIGHT_ROUND steps, so flights of different lengths
+// keep a warp full.  The counters are what that spares: an addition per warp
+// and round to the fetch cursor and to each vertex counter complete one after
+// the other, 0.8 ns each (256^3 grid, 512 x 512 x 16 paths, five depths:
+// 894 -> 727 us; refills at 1, 4, 8, 12, 16 lanes 732, 729, 727, 726, 728).
+// Issuing a round's density loads before the first is used, as
+// k_medium_transmit does, does not pay here (753 us: what is drawn past a
+// collision is lost).  The adjoint adds the pending Lambert weight gradient of
+// the previous vertex and the free-flight gradients.
 constexpr int FLIGHT_ROUND = 4;
+constexpr int FLIGHT_REFILL = 8;
 constexpr int FLIGHT_BLOCKS_PER_SM = 4;
 
 template <int MODE>
@@ -257,7 +252,7 @@ __global__ void __launch_bounds__(256) k_medium_flight(DeviceScene S, MediumGrid
     const float4* __restrict__ q = W.rays[depth & 1];
     const unsigned full = 0xffffffffu;
     const uint32_t lane = lane_id();
-    bool have = false, exhausted = false, fin = false, scatter = false, ovf = false;
+    bool have = false, fin = false, scatter = false, ovf = false;
     uint32_t idx = 0, pid = 0, seed = 0, lookups = 0;
     int32_t prim = HIT_NONE;
     int steps = 0;
@@ -265,16 +260,31 @@ __global__ void __launch_bounds__(256) k_medium_flight(DeviceScene S, MediumGrid
     f3 delta = splat(0.0f), Lrem = splat(0.0f);
     float t = 0.0f, tb = 0.0f, ts = 0.0f;
     float g_albedo = 0.0f;
+    __shared__ uint32_t s_first_end;
+    TraceShare share(count, 4u, &s_first_end);
     for (;;) {
-        const bool want = !have && !exhausted;
-        const unsigned m = __ballot_sync(full, want);
-        if (m) {
-            const int leader = __ffs(m) - 1;
-            uint32_t base = 0;
-            if ((int)lane == leader) base = atomicAdd(fetch, (uint32_t)__popc(m));
-            base = __shfl_sync(full, base, leader);
-            if (want) {
-                idx = base + (uint32_t)__popc(m & ((1u << lane) - 1u));
+        const unsigned m = __ballot_sync(full, !have || fin);
+        if (m == full || (__popc(m) >= FLIGHT_REFILL && share.more(count))) {
+            const bool push_m = have && scatter && !is_zero(beta) && fin;
+            const bool push_s = have && !scatter && prim != HIT_NONE && !is_zero(beta) && fin;
+            const uint32_t ms = claim_slot(push_m, &W.ctr[CTR_MVERT + depth]);
+            if (push_m) {
+                float4* e = verts + 3 * (size_t)ms;
+                e[0] = f4(x, __uint_as_float(pid));
+                e[1] = f4(d, __uint_as_float(seed));
+                e[2] = f4(beta, 0.0f);
+            }
+            const uint32_t ss = claim_slot(push_s, &W.ctr[CTR_SVERT + depth]);
+            if (push_s) {
+                float4* e = verts + 3 * (size_t)(capacity - 1u - ss);
+                e[0] = f4(o + ts * d, __uint_as_float(pid));
+                e[1] = f4(d, __uint_as_float(seed));
+                e[2] = f4(beta, __int_as_float(prim));
+            }
+            if (fin) have = false;
+            if (!share.more(count)) break;
+            idx = share.take(count, (uint32_t)__popc(m), (uint32_t)__popc(m & ((1u << lane) - 1u)), fetch);
+            if (!have) {
                 if (idx < count) {
                     const float4 q0 = __ldg(&q[3 * (size_t)idx]);
                     const float4 q1 = __ldg(&q[3 * (size_t)idx + 1]);
@@ -306,12 +316,10 @@ __global__ void __launch_bounds__(256) k_medium_flight(DeviceScene S, MediumGrid
                         t = ta;
                     }
                     have = true;
-                } else {
-                    exhausted = true;
                 }
             }
+            continue;
         }
-        if (!__ballot_sync(full, have)) break;
         if (have && !fin) {
             for (int r = 0; r < FLIGHT_ROUND; ++r) {
                 if (steps++ == MEDIUM_MAX_EVENTS) {
@@ -359,24 +367,6 @@ __global__ void __launch_bounds__(256) k_medium_flight(DeviceScene S, MediumGrid
                 }
             }
         }
-        const bool done = have && fin;
-        const bool push_m = done && scatter && !is_zero(beta);
-        const bool push_s = done && !scatter && prim != HIT_NONE && !is_zero(beta);
-        const uint32_t ms = claim_slot(push_m, &W.ctr[CTR_MVERT + depth]);
-        if (push_m) {
-            float4* e = verts + 3 * (size_t)ms;
-            e[0] = f4(x, __uint_as_float(pid));
-            e[1] = f4(d, __uint_as_float(seed));
-            e[2] = f4(beta, 0.0f);
-        }
-        const uint32_t ss = claim_slot(push_s, &W.ctr[CTR_SVERT + depth]);
-        if (push_s) {
-            float4* e = verts + 3 * (size_t)(capacity - 1u - ss);
-            e[0] = f4(o + ts * d, __uint_as_float(pid));
-            e[1] = f4(d, __uint_as_float(seed));
-            e[2] = f4(beta, __int_as_float(prim));
-        }
-        if (done) have = false;
     }
     if (ovf) atomicAdd(err, 1u);
     if (stats) {
@@ -393,7 +383,10 @@ __global__ void __launch_bounds__(256) k_medium_flight(DeviceScene S, MediumGrid
 
 // Medium vertices: the light term (phase function; its ratio tracking runs
 // later, in k_medium_transmit) and the phase-function sample of the next ray.
-__global__ void __launch_bounds__(256) k_medium_scatter(DeviceScene S, MediumParams P, Workspace W,
+// Latency bound (the light's loads, the queue counters): four blocks per SM in
+// one wave, 700 -> 585 us for the 512 x 512 x 16 paths above; slots claimed per
+// warp instead of per block 887.
+__global__ void __launch_bounds__(256, 4) k_medium_scatter(DeviceScene S, MediumParams P, Workspace W,
                                                         const float4* __restrict__ verts,
                                                         float4* __restrict__ shadow_aux, uint32_t depth) {
     const uint32_t count = W.ctr[CTR_MVERT + depth];
@@ -552,11 +545,16 @@ __global__ void __launch_bounds__(256, 3) k_medium_surface(DeviceScene S, Medium
 }
 
 // Ratio-tracked transmittance of the depth's shadow rays, multiplied into
-// their light terms (C = T * C).  Persistent: a lane takes the next shadow
-// ray as soon as its own is done (one atomicAdd per warp for all lanes that
-// need one) and every lane advances in rounds of TRANSMIT_ROUND steps, so a
-// warp stays full although the rays' step counts differ.
+// their light terms (C = T * C).  Persistent: lanes that are done take the
+// next shadow rays (TraceShare), TRANSMIT_REFILL or more at a time, and every
+// lane advances in rounds of TRANSMIT_ROUND steps, so a warp stays full
+// although the rays' step counts differ.  1331 -> 1135 us for the
+// 512 x 512 x 16 paths of k_medium_flight over claims from the counter for
+// every lane by itself (refills at 1, 4, 8, 12 lanes 1142, 1135, 1138, 1164).
 constexpr int TRANSMIT_ROUND = 8;
+constexpr int TRANSMIT_REFILL = 4;
+constexpr int REPLAY_REFILL = 8;
+constexpr int REPLAY_BLOCKS_PER_SM = 4;
 constexpr int TRANSMIT_BLOCKS_PER_SM = 6;
 
 __global__ void __launch_bounds__(256) k_medium_transmit(MediumGrid G, Workspace W,
@@ -566,22 +564,22 @@ __global__ void __launch_bounds__(256) k_medium_transmit(MediumGrid G, Workspace
     uint32_t* fetch = &W.ctr[CTR_TFETCH + depth];
     const unsigned full = 0xffffffffu;
     const uint32_t lane = lane_id();
-    bool have = false, exhausted = false, ovf = false;
+    bool have = false, ovf = false;
     uint32_t idx = 0, seed = 0, lookups = 0;
     int steps = 0;
     f3 o = splat(0.0f), d = splat(0.0f);
     float t = 0.0f, tb = 0.0f, T = 1.0f;
+    __shared__ uint32_t s_first_end;
+    TraceShare share(count, 4u, &s_first_end);
     for (;;) {
-        const bool want = !have && !exhausted;
-        const unsigned m = __ballot_sync(full, want);
-        if (m) {
-            const int leader = __ffs(m) - 1;
-            uint32_t base = 0;
-            if ((int)lane == leader) base = atomicAdd(fetch, (uint32_t)__popc(m));
-            base = __shfl_sync(full, base, leader);
-            if (want) {
-                idx = base + (uint32_t)__popc(m & ((1u << lane) - 1u));
-                if (idx < count) {
+        const unsigned m = __ballot_sync(full, !have);
+        if (m == full || (__popc(m) >= TRANSMIT_REFILL && share.more(count))) {
+            if (!share.more(count)) break;
+            const uint32_t i =
+                share.take(count, (uint32_t)__popc(m), (uint32_t)__popc(m & ((1u << lane) - 1u)), fetch);
+            if (!have) {
+                if (i < count) {
+                    idx = i;
                     const float4 e0 = W.shadow[3 * (size_t)idx], e1 = W.shadow[3 * (size_t)idx + 1];
                     o = xyz(e0);
                     d = xyz(e1);
@@ -597,12 +595,10 @@ __global__ void __launch_bounds__(256) k_medium_transmit(MediumGrid G, Workspace
                         tb = 0.0f;
                     }
                     have = true;
-                } else {
-                    exhausted = true;
                 }
             }
+            continue;
         }
-        if (!__ballot_sync(full, have)) break;
         if (have) {
             // A ratio-tracking point's position depends on the random step
             // lengths only, never on a density, so the round's density loads
@@ -654,50 +650,140 @@ __global__ void __launch_bounds__(256) k_medium_transmit(MediumGrid G, Workspace
 }
 
 // Shadow rays of the gradient pipeline.  LSUM: visible light terms join
-// the path's double radiance sum.  ADJOINT: for every visible shadow ray,
-// replay its ratio tracking for the density gradient, add the light (and
-// Lambert albedo) gradients, and take the term out of the path's remaining
-// radiance.
+// the path's double radiance sum.  ADJOINT: they are marked for
+// k_medium_replay.
 template <int MODE>
-__global__ void __launch_bounds__(PT_TRACE_THREADS) k_medium_connect(DeviceScene S, MediumGrid G, MediumParams P,
-                                                                     MediumBatch B, Workspace W,
-                                                                     const float4* __restrict__ shadow_aux,
-                                                                     uint32_t depth, double* __restrict__ lsum,
-                                                                     const float* __restrict__ grad_img,
-                                                                     float* g_grid, float* g_params, uint32_t np_smem,
-                                                                     uint32_t* err) {
-    extern __shared__ float s_params[];
+__global__ void __launch_bounds__(PT_TRACE_THREADS) k_medium_connect(DeviceScene S, Workspace W, uint32_t depth,
+                                                                     double* __restrict__ lsum) {
     __shared__ __align__(8) char s_stack[LaneStack<true, PT_TRACE_THREADS>::NEAR];
-    float* gp = params_begin(s_params, np_smem, g_params);
-    bool ovf = false;
     persistent_trace<true, false, PT_TRACE_THREADS>(
         S, W.shadow, 3, W.ctr[CTR_SHADOW + depth], &W.ctr[CTR_CFETCH + depth], s_stack,
         &W.err[ERR_STACK], W.stats, [&](uint32_t idx, const TravState& s) {
             if (s.hit) return;
-            const float4* e = W.shadow + 3 * (size_t)idx;
-            const float4 e0 = __ldg(e), e1 = __ldg(e + 1), e2 = __ldg(e + 2);
-            const uint32_t pid = __float_as_uint(e1.w);
-            const f3 C = xyz(e2);
-            if (MODE == LSUM) {
-                lsum_add(lsum, pid, C, 1.0);
-                return;
-            }
-            const float4 ax = __ldg(&shadow_aux[idx]);
-            const f3 delta = pixel_delta(grad_img, pid % B.pixels, P.spp);
-            uint32_t seed_ratio = __float_as_uint(ax.x);
-            uint32_t replayed = 0;
-            ratio_track(G, xyz(e0), xyz(e1), e0.w, seed_ratio, g_grid, dot3(delta, C), ovf, replayed);
-            const uint32_t li = __float_as_uint(ax.y), lam = __float_as_uint(ax.z);
-            const f3 R = __ldg(&S.lights[li].pos).w == 0.0f ? xyz(__ldg(&S.lights[li].I))
-                                                             : xyz(__ldg(&S.lights[li].L));
-            add_albedo_grad(gp + medium_light_offset(S.n_objects) + 3 * li, delta, C, R);
-            if (lam != 0u) {
-                const MatView m = load_material(S.materials, __float_as_int(__ldg(&S.objects[lam - 1u].hi).w));
-                add_albedo_grad(gp + 1 + 3 * (lam - 1u), delta, C, m.albedo_d);
-            }
-            lsum_add(lsum, pid, C, -1.0);
+            float4* e = W.shadow + 3 * (size_t)idx;
+            if (MODE == LSUM) lsum_add(lsum, __float_as_uint(e[1].w), xyz(e[2]), 1.0);
+            else e[2].w = 1.0f;  // k_medium_transmit left 0
         });
+}
+
+// ADJOINT, for every visible shadow ray: replays its ratio tracking for the
+// density gradient (-1 / (sigma_bar - sigma_v) per tracked point), adds the
+// light (and Lambert albedo) gradients, and takes the term out of the path's
+// remaining radiance.  Persistent lanes as in k_medium_transmit: inside
+// k_medium_connect the replay held up the lanes of the warp that were still
+// on their way through the tree (128^3 grid, 256 x 256 x 16 paths, five
+// depths: 1168 us there, 216 + 650 here).
+__global__ void __launch_bounds__(256, REPLAY_BLOCKS_PER_SM) k_medium_replay(DeviceScene S, MediumGrid G, MediumParams P, MediumBatch B,
+                                                       Workspace W, const float4* __restrict__ shadow_aux,
+                                                       uint32_t depth, double* __restrict__ lsum,
+                                                       const float* __restrict__ grad_img, float* g_grid,
+                                                       float* g_params, uint32_t np_smem, uint32_t* err) {
+    extern __shared__ float s_params[];
+    float* gp = params_begin(s_params, np_smem, g_params);
+    const uint32_t count = W.ctr[CTR_SHADOW + depth];
+    uint32_t* fetch = &W.ctr[CTR_RFETCH + depth];
+    const unsigned full = 0xffffffffu;
+    const uint32_t lane = lane_id();
+    bool have = false, ovf = false;
+    uint32_t seed = 0;
+    int steps = 0;
+    f3 o = splat(0.0f), d = splat(0.0f);
+    float t = 0.0f, tb = 0.0f, scale = 0.0f;
+    // The gradient of the light a lane last sampled stays in registers: every
+    // entry adds to one of a few lights, and shared-memory atomics on one
+    // address run one after the other (921 us in all with them, 650 without).
+    constexpr uint32_t NO_LIGHT = 0xffffffffu;
+    float* gl = gp + medium_light_offset(S.n_objects);
+    uint32_t acc_light = NO_LIGHT;
+    f3 acc = splat(0.0f);
+    __shared__ uint32_t s_first_end;
+    TraceShare share(count, 4u, &s_first_end);
+    for (;;) {
+        const unsigned m = __ballot_sync(full, !have);
+        if (m == full || (__popc(m) >= REPLAY_REFILL && share.more(count))) {
+            if (!share.more(count)) break;
+            const uint32_t i =
+                share.take(count, (uint32_t)__popc(m), (uint32_t)__popc(m & ((1u << lane) - 1u)), fetch);
+            if (!have && i < count) {
+                const float4* e = W.shadow + 3 * (size_t)i;
+                const float4 e2 = __ldg(e + 2);
+                if (e2.w != 0.0f) {
+                    const float4 e0 = __ldg(e), e1 = __ldg(e + 1), ax = __ldg(&shadow_aux[i]);
+                    const uint32_t pid = __float_as_uint(e1.w);
+                    const f3 C = xyz(e2), delta = pixel_delta(grad_img, pid % B.pixels, P.spp);
+                    o = xyz(e0);
+                    d = xyz(e1);
+                    seed = __float_as_uint(ax.x);
+                    scale = dot3(delta, C);
+                    steps = 0;
+                    float ta;
+                    if (box_interval(G, o, d, ta, tb)) {
+                        tb = fminf(tb, e0.w);
+                        t = ta;
+                        have = true;
+                    }
+                    const uint32_t li = __float_as_uint(ax.y), lam = __float_as_uint(ax.z);
+                    const f3 R = __ldg(&S.lights[li].pos).w == 0.0f ? xyz(__ldg(&S.lights[li].I))
+                                                                     : xyz(__ldg(&S.lights[li].L));
+                    if (li != acc_light) {
+                        if (acc_light != NO_LIGHT) add_params(gl + 3 * acc_light, acc);
+                        acc_light = li;
+                        acc = splat(0.0f);
+                    }
+                    acc = acc + albedo_grad(delta, C, R);
+                    if (lam != 0u) {
+                        const MatView mv =
+                            load_material(S.materials, __float_as_int(__ldg(&S.objects[lam - 1u].hi).w));
+                        add_albedo_grad(gp + 1 + 3 * (lam - 1u), delta, C, mv.albedo_d);
+                    }
+                    lsum_add(lsum, pid, C, -1.0);
+                }
+            }
+            continue;
+        }
+        if (have) {
+            // the round's density loads are all issued before the first is used
+            float sk[TRANSMIT_ROUND];
+            uint32_t vk[TRANSMIT_ROUND];
+            bool in[TRANSMIT_ROUND];
+            bool done = false;
+#pragma unroll
+            for (int r = 0; r < TRANSMIT_ROUND; ++r) {
+                in[r] = false;
+                sk[r] = 0.0f;
+                vk[r] = 0u;
+                if (done) continue;
+                if (steps++ == MEDIUM_MAX_EVENTS) {
+                    ovf = done = true;
+                    continue;
+                }
+                t += free_step(G, seed);
+                if (!(t < tb)) {
+                    done = true;
+                    continue;
+                }
+                in[r] = true;
+                vk[r] = voxel_of(G, o + t * d);
+                sk[r] = __ldg(&G.density[vk[r]]);
+            }
+#pragma unroll
+            for (int r = 0; r < TRANSMIT_ROUND; ++r)
+                if (in[r]) atomicAdd(&g_grid[vk[r]], -scale / (G.majorant - sk[r]));
+            if (done) have = false;
+        }
+    }
     if (ovf) atomicAdd(err, 1u);
+    // all of the warp's lanes on one light (as a rule): one sum for the warp
+    int same;
+    __match_all_sync(full, acc_light, &same);
+    if (same) {
+        for (int off = 16; off > 0; off >>= 1) {
+            acc.x += __shfl_down_sync(full, acc.x, off);
+            acc.y += __shfl_down_sync(full, acc.y, off);
+            acc.z += __shfl_down_sync(full, acc.z, off);
+        }
+    }
+    if (acc_light != NO_LIGHT && (!same || lane == 0)) add_params(gl + 3 * acc_light, acc);
     params_end(s_params, np_smem, g_params);
 }
 
@@ -745,7 +831,6 @@ cudaError_t wavefront(const DeviceScene& S, const MediumGrid& G, const MediumPar
                       int num_sms, cudaStream_t st, Mark mark) {
     const uint32_t np = medium_param_count(S.n_objects, S.n_lights);
     const uint32_t np_smem = MODE == ADJOINT && np <= MEDIUM_SMEM_PARAMS ? np : 0;
-    const int connect_smem = (int)(np_smem * sizeof(float));
     unsigned long long* stats = MODE == RENDER ? W.stats : nullptr;
     cudaError_t e = cudaMemsetAsync(W.pt.ctr, 0, sizeof(uint32_t) * CTR_TOTAL, st);
     if (e != cudaSuccess) return e;
@@ -757,7 +842,7 @@ cudaError_t wavefront(const DeviceScene& S, const MediumGrid& G, const MediumPar
         mark();
         k_medium_flight<MODE><<<num_sms * FLIGHT_BLOCKS_PER_SM, 256, np_smem * sizeof(float), st>>>(
             S, G, P, B, W.pt, W.verts, W.capacity, d, W.lsum, grad_img, g_grid, g_params, np_smem, err, stats);
-        k_medium_scatter<<<num_sms * 8, 256, 0, st>>>(S, P, W.pt, W.verts, W.shadow_aux, d);
+        k_medium_scatter<<<num_sms * 4, 256, 0, st>>>(S, P, W.pt, W.verts, W.shadow_aux, d);
         k_medium_surface<MODE><<<num_sms * 8, 256, np_smem * sizeof(float), st>>>(
             S, P, B, W.pt, W.verts, W.capacity, W.shadow_aux, d, W.lsum, grad_img, g_params, np_smem);
         mark();
@@ -766,8 +851,11 @@ cudaError_t wavefront(const DeviceScene& S, const MediumGrid& G, const MediumPar
         if constexpr (MODE == RENDER) {
             if ((e = pt_launch_connect(S, W.pt, d, num_sms, st)) != cudaSuccess) return e;
         } else {
-            k_medium_connect<MODE><<<num_sms * W.pt.trace_blocks_per_sm, PT_TRACE_THREADS, connect_smem, st>>>(
-                S, G, P, B, W.pt, W.shadow_aux, d, W.lsum, grad_img, g_grid, g_params, np_smem, err);
+            k_medium_connect<MODE>
+                <<<num_sms * W.pt.trace_blocks_per_sm, PT_TRACE_THREADS, 0, st>>>(S, W.pt, d, W.lsum);
+            if constexpr (MODE == ADJOINT)
+                k_medium_replay<<<num_sms * REPLAY_BLOCKS_PER_SM, 256, np_smem * sizeof(float), st>>>(
+                    S, G, P, B, W.pt, W.shadow_aux, d, W.lsum, grad_img, g_grid, g_params, np_smem, err);
         }
         mark();
     }
