@@ -155,7 +155,9 @@ __device__ __forceinline__ uint32_t vol_class(const DeviceScene& S, float2 h) {
 // queue entry.  4 blocks per SM (64 registers, with spills): latency bound, so
 // the warps weigh more than the spills (512 x 512 x 32 frames, 5 depths, B200: 2
 // blocks 6.4 ms, 3 5.9, 4 5.6, 5 5.9; paths inside a mesh apart from those inside
-// a sphere 5.6 -> 5.3).
+// a sphere 5.6 -> 5.3; one copy of the light sample, of the direction sample and
+// of their callers for all kinds of vertex, 288 bytes of stack, 5.3 -> 4.1, then
+// 3 or 5 blocks 4.5, 4.7).
 __global__ void __launch_bounds__(256, 4) k_vol_shade(const __grid_constant__ DeviceScene S, PTFrame F, Workspace W,
                                                       uint32_t depth) {
     const uint32_t n_out = W.ctr[CTR_RAYS + depth], n_in = W.ctr[CTR_VOL_INSIDE + depth];
@@ -253,91 +255,87 @@ __global__ void __launch_bounds__(256, 4) k_vol_shade(const __grid_constant__ De
                     vsa = im.sigma_a;
                     vg = im.g;
                 }
-                bool handled = false, stop = false;
-                {
-                    const f3 st = vsa + vss;
-                    const uint32_t ch = (uint32_t)(rnd(seed) * 3.0f);
-                    if (!feq0(comp(st, ch))) {
-                        const float t = -logf(1.0f - rnd(seed)) / comp(st, ch);
-                        if (t < g.t) {
-                            handled = true;
-                            const f3 Pe = o + t * d;
-                            const float sp = comp(vss, ch) / comp(st, ch);
-                            if (rnd(seed) < sp) {
-                                float pdf = 0.0f;
-                                for (uint32_t k = 0; k < 3; ++k) pdf += comp(st, k) * expf(-1.0f * comp(st, k) * t);
-                                pdf /= 3.0f;
-                                rw = rw * vss / sp * vexp(-1.0f * st * t) / pdf;
-                                f3 ldir;
-                                float dist;
-                                const f3 lrad = sample_nee(S, m, seed, Pe, inc, g.N, ldir, dist);
-                                f3 att = splat(1.0f);
-                                f3 so = Pe + 0.001f * ldir;
-                                if (inside) {
-                                    float te;
-                                    f3 Ne;
-                                    f3 ePs = Pe;
-                                    if (!trace_object(S, obj_index, Pe, normalize(ldir), te, Ne)) te = 0.0f;
-                                    else ePs = Pe + te * normalize(ldir);
-                                    att = vexp(-1.0f * st * te) * hg_phase(vg, -dot(inc, ldir));
-                                    so = ePs + 0.001f * ldir;
-                                    dist -= te;
-                                } else if (F.estimator) {
-                                    att = splat(hg_phase(vg, -dot(inc, ldir)));
-                                }
-                                const f3 sst = scene_sa + scene_ss;
-                                const f3 c = nl * vexp(-1.0f * sst * fminf(dist, 100000000.0f)) * att * lrad * rw;
-                                push_sh = !is_zero(c);  // a zero term changes no sum
-                                sh0 = f4(so, dist);
-                                sh1 = f4(normalize(ldir), __uint_as_float(pid));
-                                sh2 = f4(c, 0.0f);
-                                const float4 shg = sample_hg(vg, -1.0f * inc, seed);
-                                out_dir = xyz(shg);
-                                ray_start = Pe;
-                                next_valid = true;
-                            } else {
-                                rw = splat(0.0f);
-                            }
-                        } else {
-                            float pdf = 0.0f;
-                            for (uint32_t k = 0; k < 3; ++k) pdf += expf(-comp(st, k) * g.t);
-                            pdf /= 3.0f;
-                            rw = rw * vexp(-1.0f * st * g.t) / pdf;
-                            ray_start = g.P;
+                // What happens along the ray: a scattering event in the volume
+                // (EVENT), the surface seen from its front (FRONT), from behind
+                // (BACK) or a VOLUME interface.  One copy of the light sample
+                // serves EVENT and FRONT, one of the direction sample the other
+                // three: the kernel's code does not fit the instruction caches,
+                // and its warps meet again there.
+                enum : int { NOTHING, EVENT, FRONT, BACK, INTERFACE };
+                int kind = m.type == 5 ? INTERFACE : m.type != 3 && dot(g.N, inc) <= 0.0f ? BACK : FRONT;
+                bool stop = false;
+                ray_start = g.P;
+                const f3 st = vsa + vss;
+                const uint32_t ch = (uint32_t)(rnd(seed) * 3.0f);
+                if (!feq0(comp(st, ch))) {
+                    float t = -logf(1.0f - rnd(seed)) / comp(st, ch);
+                    const bool event = t < g.t;
+                    float sp = 1.0f;
+                    if (event) {
+                        sp = comp(vss, ch) / comp(st, ch);
+                        kind = rnd(seed) < sp ? EVENT : NOTHING;
+                    } else {
+                        t = g.t;
+                    }
+                    if (kind == NOTHING) {
+                        rw = splat(0.0f);
+                    } else {
+                        float pdf = 0.0f;
+                        for (uint32_t k = 0; k < 3; ++k) {
+                            const float e = expf(-comp(st, k) * t);
+                            pdf += event ? comp(st, k) * e : e;
                         }
+                        pdf /= 3.0f;
+                        if (event) rw = rw * vss / sp;
+                        rw = rw * vexp(-1.0f * st * t) / pdf;
+                        if (event) ray_start = o + t * d;
                     }
                 }
-                if (!handled) {
-                    if (m.type == 5) {  // VOLUME interface (VolumeRenderer.cu:269-278)
-                        out_dir = xyz(sample_direction(m, seed, inc, g.N));
-                        ray_start = g.P;
-                        const bool refl = dot(inc, g.N) * dot(out_dir, g.N) > 0.0f;
+                if (kind == EVENT || kind == FRONT) {
+                    f3 ldir, x;
+                    float dist, scale = nl;
+                    const f3 lrad = sample_nee(S, m, seed, ray_start, inc, g.N, ldir, dist);
+                    f3 from = ray_start, sst = st;
+                    if (kind == EVENT) {
+                        sst = scene_sa + scene_ss;
+                        x = splat(1.0f);
+                        if (inside) {
+                            float te;
+                            f3 Ne;
+                            if (!trace_object(S, obj_index, ray_start, normalize(ldir), te, Ne)) te = 0.0f;
+                            else from = ray_start + te * normalize(ldir);
+                            x = vexp(-1.0f * st * te) * hg_phase(vg, -dot(inc, ldir));
+                            dist -= te;
+                        } else if (F.estimator) {
+                            x = splat(hg_phase(vg, -dot(inc, ldir)));
+                        }
+                    } else {
+                        scale = nl * fmaxf(0.0f, dot(g.N, ldir));
+                        x = brdf(m, inc, ldir, g.N);
+                    }
+                    const f3 c = scale * vexp(-1.0f * sst * fminf(dist, 100000000.0f)) * x * lrad * rw;
+                    push_sh = !is_zero(c);  // a zero term changes no sum
+                    sh0 = f4(from + 0.001f * ldir, dist);
+                    sh1 = f4(normalize(ldir), __uint_as_float(pid));
+                    sh2 = f4(c, 0.0f);
+                }
+                if (kind == EVENT) {
+                    out_dir = xyz(sample_hg(vg, -1.0f * inc, seed));
+                    next_valid = true;
+                } else if (kind != NOTHING) {
+                    if (kind == BACK) rw = splat(0.0f);
+                    const float4 sd = sample_direction(m, seed, inc, g.N);
+                    const f3 dir = xyz(sd);
+                    if (kind == INTERFACE) {  // VolumeRenderer.cu:269-278
+                        const bool refl = dot(inc, g.N) * dot(dir, g.N) > 0.0f;
                         inside = refl ? inside : !inside;
                         obj_index = g.obj;
+                        out_dir = dir;
                         next_valid = true;
-                    } else {
-                        if (m.type != 3 && dot(g.N, inc) <= 0.0f) {
-                            rw = splat(0.0f);
-                        } else {
-                            f3 ldir;
-                            float dist;
-                            const f3 lrad = sample_nee(S, m, seed, g.P, inc, g.N, ldir, dist);
-                            const f3 c = nl * fmaxf(0.0f, dot(g.N, ldir)) *
-                                         vexp(-1.0f * (vss + vsa) * fminf(dist, 100000000.0f)) *
-                                         brdf(m, inc, ldir, g.N) * lrad * rw;
-                            push_sh = !is_zero(c);  // a zero term changes no sum
-                            sh0 = f4(g.P + 0.001f * ldir, dist);
-                            sh1 = f4(normalize(ldir), __uint_as_float(pid));
-                            sh2 = f4(c, 0.0f);
-                        }
-                        const float4 sd = sample_direction(m, seed, inc, g.N);
-                        const f3 dir = xyz(sd);
-                        if (!(norm(dir) == 0.0f)) {
-                            rw = rw * fabsf(dot(dir, g.N)) * brdf(m, inc, dir, g.N) / sd.w;
-                            out_dir = dir;
-                            ray_start = g.P;
-                            next_valid = true;
-                        }
+                    } else if (!(norm(dir) == 0.0f)) {
+                        rw = rw * fabsf(dot(dir, g.N)) * brdf(m, inc, dir, g.N) / sd.w;
+                        out_dir = dir;
+                        next_valid = true;
                     }
                     if (F.use_rr) {
                         const float alpha = clampf(fmaxf(rw.x, fmaxf(rw.y, rw.z)), 0.0f, 1.0f);
