@@ -497,9 +497,9 @@ __global__ void __launch_bounds__(256, 4) k_gd_shade(const __grid_constant__ Dev
                 if (!SHIFT) valid[j] |= 1ull << depth;
                 const f3 inc = -1.0f * d;
                 const MatView m = object_material(S, g.obj);
-                {
+                const f3 e = rw * m.albedo_e;
+                if (!is_zero(e)) {
                     float4 r = W.radiance[pid];
-                    const f3 e = rw * m.albedo_e;
                     r.x += e.x; r.y += e.y; r.z += e.z;
                     W.radiance[pid] = r;
                 }
