@@ -218,21 +218,18 @@ __device__ __forceinline__ void shade_one(const DeviceScene& S, const PTFrame& F
                                           const CacheFrame& C, uint32_t depth, const float4& q0, const float4& q1,
                                           const float4& q2, float2 h, ShadeOut& so, const TexRecord& R = TexRecord{}) {
     const uint32_t pid = __float_as_uint(q0.w);
-    if (!CACHE && !REC) {
-        // most vertices emit nothing: the path's radiance, a sector of its own in
-        // late depths, is read and written only for a nonzero term (16.8 M paths
-        // of the Cornell box 10.37 -> 9.84 ms)
-        f3 add = splat(0.0f);
-        shade_core<CACHE, PHYS>(S, F, C, depth, q0, q1, q2, h, add, so);
-        if (!is_zero(add)) {
-            const f3 rad = xyz(NC ? W.radiance[pid] : __ldcg(&W.radiance[pid])) + add;
-            W.radiance[pid] = f4(rad, 0.0f);
-        }
-        return;
-    }
-    f3 rad = xyz(NC ? W.radiance[pid] : __ldcg(&W.radiance[pid]));
+    // Most vertices emit nothing: the path's radiance, a sector of its own in
+    // late depths, is read and written only for a nonzero term (16.8 M paths of
+    // the Cornell box 10.37 -> 9.84 ms).  Training paths of a cached frame record
+    // it at every vertex.
+    const bool always = CACHE && C.train_stride != 0 && pid % C.train_stride == C.train_phase;
+    f3 rad = splat(0.0f);
+    if (always) rad = xyz(W.radiance[pid]);
     shade_core<CACHE, PHYS>(S, F, C, depth, q0, q1, q2, h, rad, so);
-    W.radiance[pid] = f4(rad, 0.0f);
+    const bool changed = always || !is_zero(rad);
+    if (!always && (changed || (REC && so.texel >= 0)))
+        rad = xyz(NC ? W.radiance[pid] : __ldcg(&W.radiance[pid])) + rad;
+    if (changed) W.radiance[pid] = f4(rad, 0.0f);
     if (REC && so.texel >= 0) {
         R.vertex[(size_t)depth * R.stride + pid] = f4(rad, __int_as_float(so.texel));
         R.depths[pid] |= 1u << depth;
