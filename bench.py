@@ -1311,15 +1311,15 @@ def run_method(args) -> int:
                 "gpu_launches": ((2 + 3 * DEPTH) * -(-args.steps // max(1, BATCH_PATHS // (W * H)))
                                  if args.scene == "volume" else
                                  2 * (1 + 3 * DEPTH) * -(-args.steps // max(1, BATCH_PATHS // (5 * W * H)))
-                                 + 52 * args.steps),
+                                 + 12 * args.steps),
                 "device_errors": r.error_count(), "clocks": clocks}
         if rec_ms is not None:
             rec_bytes = 72.0 * W * H * 50 + 72.0 * W * H  # 50 passes of 5 reads + 1 write, init 6 reads + 3 writes
             line["roofline_reconstruction"] = {
-                "kernel": "k_gdpt_init + 10 x k_gdpt_opt_blocked (5 passes each)", "ms_per_step": rec_ms / args.steps,
+                "kernel": "k_gdpt_init + 10 x k_gdpt_opt (5 passes each)", "ms_per_step": rec_ms / args.steps,
                 "achieved": rec_bytes * args.steps / (rec_ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                 "frac": rec_bytes * args.steps / (rec_ms * 1e-3) / 1e9 / peak,
-                "note": "algorithmic 72 B per pixel and pass (50 passes); the blocked kernel reads each image once per 5 passes, and the nine 3 MB images stay in L2"}
+                "note": "algorithmic 72 B per pixel and pass (50 passes); the kernel reads each image once per 5 passes, and the nine 3 MB images stay in L2"}
         if world == 1 and not args.no_reference_cuda:
             try:
                 from oracle import bridge
@@ -1423,9 +1423,9 @@ def run_post(args) -> int:
     peak, peak_src = 6650.0, "fallback"
     if os.path.exists(peaks_path):
         peak, peak_src = float(json.load(open(peaks_path))["hbm_gbs"]), "measured"
-    # k_bloom_down: 12 B read + 3 B written per pixel (half resolution);
-    # k_bloom_up fused with the tone map: 12 + 3 B read, 4 B written
-    bytes_px = 12.0 + 3.0 + 12.0 + 3.0 + 4.0
+    # k_bloom fused with the tone map: 12 B read, 4 B written per pixel (the
+    # half-resolution level stays in shared memory)
+    bytes_px = 12.0 + 4.0
     achieved = bytes_px * W * H * args.steps / (ms * 1e-3) / 1e9
     if rank == 0:
         line = {"metric": cfg["metric"], "value": value, "unit": "Mpixels/s", "n_gpus": world, "steps": args.steps,
@@ -1440,8 +1440,8 @@ def run_post(args) -> int:
                         "note": "HDR upload + bloom/tone map + RGBA8 readback per step"},
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                              "frac": achieved / peak, "traffic": None, "peak_source": f"{peak_src} hbm_gbs",
-                             "kernel": "k_bloom_down + k_bloom_up (fused tone map)", "bytes_per_pixel": bytes_px},
-                "gpu_launches": 2 * args.steps, "clocks": clocks}
+                             "kernel": "k_bloom (fused tone map)", "bytes_per_pixel": bytes_px},
+                "gpu_launches": args.steps, "clocks": clocks}
         if world == 1 and not args.no_reference_cuda:
             try:
                 from oracle import bridge
