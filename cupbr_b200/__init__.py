@@ -380,10 +380,11 @@ class PBRenderer:
         N.call("cupbr_renderer_set_pipelined", self._h, 1 if enable else 0)
 
     def set_tail_paths(self, paths: int) -> None:
-        """Ray queues below `paths` rays (default 2^15 on one stream, off
-        when pipelined) finish their paths in one per-path launch, and so do
-        wavefronts of fewer than `paths` paths (default 3 * 2^17) from the
-        start (same image; 0 = off)."""
+        """Ray queues below `paths` rays (default 2^15; off when pipelined on
+        a stream other than the legacy one) finish their paths in one per-path
+        launch, and so do wavefronts of fewer than `paths` paths (default
+        3 * 2^17, or 3 * 2^15 when so pipelined) from the start (same image;
+        0 = off)."""
         N.call("cupbr_renderer_set_tail_paths", self._h, paths)
 
     def set_batch_paths(self, paths: int) -> None:

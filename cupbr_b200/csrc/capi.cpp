@@ -249,13 +249,18 @@ struct cupbr_renderer_s {
     // beats the stage kernels up to 3 x 2^17 paths (Cornell box, spheres, terrain
     // at 512 x 512: 334 against 402 us, 444 / 506, 875 / 1030; at 960 x 540
     // 506 / 516, 606 / 589, 1357 / 1278; at 256 x 256 138 / 255, 196 / 374,
-    // 513 / 729; eight pipelined 256 x 256 frames 1117 / 2153, 1594 / 3397,
-    // 4149 / 8085).  The end of a larger frame pays below 2^15 rays (terrain
-    // 960 x 540 1277 against 1376 us), not pipelined, where the next frame's
-    // wavefront fills the SMs that a sparse queue leaves idle.
+    // 513 / 729).  The end of a larger frame pays below 2^15 rays (terrain
+    // 960 x 540 1277 against 1376 us).  Where pipelined frames overlap, the
+    // next frames' wavefronts fill the SMs that a sparse queue leaves idle: no
+    // tail, and one launch up to 3 x 2^15 paths (us per frame of a long run,
+    // 256 x 256: 77 / 121, 103 / 138, 302 / 478; 362 x 362: 147 / 153,
+    // 172 / 150, 459 / 581; 512 x 512: 289 / 215, 330 / 181, 875 / 742).  They do
+    // not overlap on the legacy stream, which waits for the internal streams and
+    // holds them up.
     PTTail tail() const {
         if (tail_set) return {tail_paths, tail_paths};
-        return {pipelined ? 0u : 1u << 15, 3u << 17};
+        if (pipelined && stream != nullptr && stream != cudaStreamLegacy) return {0u, 3u << 15};
+        return {1u << 15, 3u << 17};
     }
     // rays of the last wavefront frame: closest-hit and shadow queue sizes
     cudaError_t read_wavefront_rays() {

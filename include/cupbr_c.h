@@ -282,11 +282,12 @@ int cupbr_renderer_render(cupbr_renderer_t r, const cupbr_camera* camera);
 int cupbr_renderer_render_frames(cupbr_renderer_t r, const cupbr_camera* camera, uint32_t nframes);
 int cupbr_renderer_set_batch_paths(cupbr_renderer_t r, uint32_t paths);
 /* PATHTRACER: once a depth's ray queue holds fewer than `paths` rays
- * (default 32,768 on one stream; off when pipelined, where the other
- * streams' frames fill the SMs a sparse queue leaves idle), one thread per
- * ray traces the rest of its path in one launch instead of a launch per
- * stage and depth.  A wavefront of fewer than `paths` paths (default 393,216,
- * pipelined or not) is that one launch whole.  Same image; 0 = off. */
+ * (default 32,768 on one stream; off when pipelined on a stream other than the
+ * legacy one, where other frames fill the SMs a sparse queue leaves idle), one
+ * thread per ray traces the rest of its path in one launch instead of a launch
+ * per stage and depth.  A wavefront of fewer than `paths` paths (default
+ * 393,216, or 98,304 when so pipelined) is that one launch whole.  Same image;
+ * 0 = off. */
 int cupbr_renderer_set_tail_paths(cupbr_renderer_t r, uint32_t paths);
 /* render_frames through one persistent-kernel launch instead of wavefronts
  * (no counterpart in the reference): each warp takes 32 pixels (an 8x4
@@ -426,8 +427,9 @@ int cupbr_postprocessor_bloom_tonemap(cupbr_postprocessor_t p, const float thres
  * (width/2)*(height/2) <= 1048576 (inputs up to 2048x2048), larger images
  * are rejected with CUPBR_ERR_ARG.  The first call on a device looks up the
  * array's device address, so make that first call before any stream
- * capture.  All calls share the one array: calls whose GPU work overlaps
- * (two streams, two host threads) race and must be ordered by the caller.
+ * capture.  Calls whose output overlaps their input use the array (the others
+ * need no scratch): such calls share it, and where their GPU work overlaps
+ * (two streams, two host threads) they race and must be ordered by the caller.
  * The looked-up address is kept per device for the life of the process; a
  * cudaDeviceReset of a device invalidates it, so a process that resets a
  * device must not call this entry point on that device afterwards. */

@@ -11,7 +11,7 @@ from cupbr_b200 import scenes
 pytestmark = pytest.mark.gpu
 
 
-def render(w, h, frames=1, tail=None, pipelined=False):
+def render(w, h, frames=1, tail=None, pipelined=False, stream=None):
     r = cb.PBRenderer(cb.RenderingMethod.PATHTRACER)
     r.set_output_size(w, h)
     r.register_scene(scenes.cornell_box().build())
@@ -20,9 +20,13 @@ def render(w, h, frames=1, tail=None, pipelined=False):
     if tail is not None:
         r.set_tail_paths(tail)
     r.set_pipelined(pipelined)
+    if stream is not None:
+        r.set_stream(stream)
     cam = cb.Camera(w, h)
     for _ in range(frames):
         r.render(cam)
+    if stream is not None:
+        stream.synchronize()
     img = r.get_output_image().numpy()
     assert r.error_count() == 0
     return img
@@ -46,3 +50,10 @@ def test_few_paths_same_image(w, h):
 @pytest.mark.parametrize("pipelined", [False, True])
 def test_default_choice_same_image(w, h, pipelined):
     assert np.array_equal(render(w, h, 3, 0), render(w, h, 3, None, pipelined))
+
+
+# the same pipelined on a stream of its own, where frames overlap
+@pytest.mark.parametrize("w,h", [(312, 315), (384, 256)])
+def test_overlapping_choice_same_image(w, h):
+    torch = pytest.importorskip("torch")
+    assert np.array_equal(render(w, h, 6, 0), render(w, h, 6, None, True, torch.cuda.Stream()))
