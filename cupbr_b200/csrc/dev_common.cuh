@@ -157,6 +157,7 @@ struct DeviceScene {
     uint32_t tex_w, tex_h;
     uint32_t sphere_base, quad_base;      // unified slot offsets (triangles start at 0)
     float4 vol_sigma_s, vol_sigma_a;      // scene medium (Scene.h:23), w = g in sigma_s
+    uint32_t mixed_materials;  // vertices of more than one shading class (shade_class; as committed, it only chooses a block size)
 };
 
 // Hit record written by the closest-hit pass: t and the primitive ref

@@ -484,6 +484,12 @@ bool commit_scene(GpuScene& g, const BvhBuildParams& params, std::string& err) {
     D.n_planes = (uint32_t)nP;
     D.n_objects = (uint32_t)nobj;
     D.n_lights = (uint32_t)sc.lights.size();
+    uint32_t classes = sc.env_w > 0 ? 1u : 0u;  // bits: misses that look up the environment, diffuse, GGX, delta
+    for (const auto& ob : sc.objects) {
+        const int type = (int)ob.mat.type;
+        classes |= type == 4 ? 4u : type == 2 || type == 3 ? 8u : 2u;
+    }
+    D.mixed_materials = (classes & (classes - 1u)) != 0u ? 1u : 0u;
     D.env_w = sc.env_w;
     D.env_h = sc.env_h;
     D.sphere_base = (uint32_t)nT;

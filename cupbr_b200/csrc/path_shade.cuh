@@ -236,31 +236,31 @@ __device__ __forceinline__ void shade_one(const DeviceScene& S, const PTFrame& F
     }
 }
 
-// The shading stage of one depth over ray queue[depth] with blocks of 256
-// threads striding over 256-ray chunks (k_shade, and the persistent batch
+// The shading stage of one depth over ray queue[depth] with blocks of T
+// threads striding over T-ray chunks (k_shade, and the persistent batch
 // kernel's shading stage): each chunk is shaded in material-class order
 // (misses, diffuse, GGX, delta), so most warps run one BSDF.  A queue below
 // C.tail_threshold is left to k_tail.
-template <bool CACHE, bool PHYS, bool NC = true, bool REC = false>
+template <bool CACHE, bool PHYS, bool NC = true, bool REC = false, uint32_t T = 256>
 __device__ __forceinline__ void shade_stage(const DeviceScene& S, const PTFrame& F, const Workspace& W, uint32_t depth,
                                             const CacheFrame& C, const TexRecord& R = TexRecord{}) {
     const uint32_t count = NC ? W.ctr[CTR_RAYS + depth] : __ldcg(&W.ctr[CTR_RAYS + depth]);
     if (count < C.tail_threshold) return;
     const float4* __restrict__ q = W.rays[depth & 1];
     float4* __restrict__ qn = W.rays[(depth + 1) & 1];
-    // each chunk of 256 rays is shaded in material-class order (misses,
+    // each chunk of T rays is shaded in material-class order (misses,
     // diffuse, GGX, delta), so most warps run one BSDF's code
-    __shared__ uint32_t s_cnt[8][4];
-    __shared__ uint32_t s_idx[256];
+    __shared__ uint32_t s_cnt[T / 32][4];
+    __shared__ uint32_t s_idx[T];
     constexpr int QUEUES = CACHE ? 3 : 2;
-    __shared__ BlockClaim<QUEUES, 8> s_claim;
+    __shared__ BlockClaim<QUEUES, T / 32> s_claim;
     const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
     const unsigned full = 0xffffffffu;
 
-    for (uint32_t c0 = blockIdx.x * 256u; c0 < count; c0 += gridDim.x * 256u) {
+    for (uint32_t c0 = blockIdx.x * T; c0 < count; c0 += gridDim.x * T) {
         const uint32_t mine = c0 + threadIdx.x;
-        if (NC && c0 + gridDim.x * 256u < count) {
-            const uint32_t n0 = c0 + gridDim.x * 256u, left = min(256u, count - n0);
+        if (NC && c0 + gridDim.x * T < count) {
+            const uint32_t n0 = c0 + gridDim.x * T, left = min(T, count - n0);
             prefetch_block(q + 3 * (size_t)n0, 48u * left);
             prefetch_block(W.hits + n0, 8u * left);
         }
@@ -277,7 +277,7 @@ __device__ __forceinline__ void shade_stage(const DeviceScene& S, const PTFrame&
         if (cls < 4) {
             uint32_t base = 0;
             for (uint32_t k = 0; k < cls; ++k)
-                for (uint32_t w = 0; w < 8; ++w) base += s_cnt[w][k];
+                for (uint32_t w = 0; w < T / 32; ++w) base += s_cnt[w][k];
             for (uint32_t w = 0; w < wid; ++w) base += s_cnt[w][cls];
             s_idx[base + rank] = mine;
         }

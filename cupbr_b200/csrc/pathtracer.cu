@@ -110,9 +110,14 @@ __global__ void __launch_bounds__(PT_TRACE_THREADS, 8) k_connect(DeviceScene S, 
 
 // 4 blocks of 256 per SM (64 registers; measured faster than the
 // unconstrained 92 registers at 2 blocks, despite a few spilled bytes).
-template <bool CACHE, bool PHYS>
-__global__ void __launch_bounds__(256, 4) k_shade(DeviceScene S, PTFrame F, Workspace W, uint32_t depth, CacheFrame C) {
-    shade_stage<CACHE, PHYS>(S, F, W, depth, C);
+// Blocks of T rays sorted by material class.  Where the materials are of
+// several classes a large block fills more warps with one class (terrain 1080p x
+// 16 frames, T = 128 / 256 / 512: 47.7, 44.5, 42.7 ms); where there is one class
+// a small block waits less at its barriers (Cornell box, 16.8 M paths: 9.67,
+// 9.82, 10.28 ms).  shade_blocks chooses.
+template <bool CACHE, bool PHYS, uint32_t T>
+__global__ void __launch_bounds__(T, 1024 / T) k_shade(DeviceScene S, PTFrame F, Workspace W, uint32_t depth, CacheFrame C) {
+    shade_stage<CACHE, PHYS, true, false, T>(S, F, W, depth, C);
 }
 
 // Tail of a frame: once ray queue[depth] holds fewer than C.tail_threshold
@@ -242,6 +247,13 @@ cudaError_t pt_launch_extend_camera(const DeviceScene& S, const Workspace& W, in
     return cudaGetLastError();
 }
 
+template <bool CACHE, bool PHYS>
+static void shade_blocks(const DeviceScene& S, const PTFrame& F, const Workspace& W, uint32_t depth,
+                         const CacheFrame& C, int num_sms, cudaStream_t st) {
+    if (S.mixed_materials) k_shade<CACHE, PHYS, 512><<<num_sms * 4, 512, 0, st>>>(S, F, W, depth, C);
+    else k_shade<CACHE, PHYS, 128><<<num_sms * 16, 128, 0, st>>>(S, F, W, depth, C);
+}
+
 // Warps of a tail kernel that fit the device at once.
 template <bool CACHE, bool PHYS>
 static uint32_t tail_warps(int num_sms) {
@@ -281,14 +293,14 @@ cudaError_t pt_launch_connect(const DeviceScene& S, const Workspace& W, uint32_t
 
 cudaError_t pt_launch_shade(const DeviceScene& S, const PTFrame& F, const Workspace& W, uint32_t depth, int num_sms,
                             cudaStream_t st) {
-    if (F.estimator) k_shade<false, true><<<num_sms * 8, 256, 0, st>>>(S, F, W, depth, CacheFrame{});
-    else k_shade<false, false><<<num_sms * 8, 256, 0, st>>>(S, F, W, depth, CacheFrame{});
+    if (F.estimator) shade_blocks<false, true>(S, F, W, depth, CacheFrame{}, num_sms, st);
+    else shade_blocks<false, false>(S, F, W, depth, CacheFrame{}, num_sms, st);
     return cudaGetLastError();
 }
 
 cudaError_t pt_shade_cached(const DeviceScene& S, const PTFrame& F, const Workspace& W, const CacheFrame& C,
                             uint32_t depth, int num_sms, cudaStream_t st) {
-    k_shade<true, false><<<num_sms * 8, 256, 0, st>>>(S, F, W, depth, C);
+    shade_blocks<true, false>(S, F, W, depth, C, num_sms, st);
     return cudaGetLastError();
 }
 
@@ -320,7 +332,6 @@ cudaError_t pt_render_frame(const DeviceScene& S, const PTFrame& F, const Worksp
     k_camera<<<nb, 256, 0, st>>>(F, W);
     mark();
     const int trace_blocks = num_sms * W.trace_blocks_per_sm;
-    const int shade_blocks = num_sms * 8;
     // instrumented frames count every ray's traversal: no tail there
     CacheFrame T{};
     const bool whole = !count_stats && F.n_paths < tail.whole_paths;
@@ -342,8 +353,8 @@ cudaError_t pt_render_frame(const DeviceScene& S, const PTFrame& F, const Worksp
         else if (d == 0) k_extend_camera<<<trace_blocks, PT_TRACE_THREADS, 0, st>>>(S, W, T.tail_threshold);
         else k_extend<false><<<trace_blocks, PT_TRACE_THREADS, 0, st>>>(S, W, d, T.tail_threshold);
         mark();
-        if (F.estimator) k_shade<false, true><<<shade_blocks, 256, 0, st>>>(S, F, W, d, T);
-        else k_shade<false, false><<<shade_blocks, 256, 0, st>>>(S, F, W, d, T);
+        if (F.estimator) shade_blocks<false, true>(S, F, W, d, T, num_sms, st);
+        else shade_blocks<false, false>(S, F, W, d, T, num_sms, st);
         mark();
         if (count_stats) k_connect<true><<<trace_blocks, PT_TRACE_THREADS, 0, st>>>(S, W, d);
         else k_connect<false><<<trace_blocks, PT_TRACE_THREADS, 0, st>>>(S, W, d);
