@@ -961,8 +961,9 @@ __global__ void k_write_nodes(const W4* __restrict__ w4, uint32_t n4, const uint
 // Centre and half extent of [lo, hi], rounded outwards: the box they span
 // holds [lo, hi], with 2^-20 of the extent to spare for the traversal's
 // arithmetic on them.  A missing child (inverted bounds) gets half extent
-// -inf, which no slab test accepts; a bound too large to carry its
-// opposite's position gets a box around the origin.
+// -inf, which slab_child turns down for every ray that walks a tree
+// (slab_walks); a bound too large to carry its opposite's position gets a box
+// around the origin.
 __device__ __forceinline__ void slab_axis(float lo, float hi, bool empty, float& c, float& h) {
     if (empty) {
         c = 0.0f;

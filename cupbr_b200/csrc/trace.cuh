@@ -17,6 +17,7 @@
 
 #include "bvh_build.hpp"
 #include "dev_common.cuh"
+#include "slab.hpp"
 
 namespace cupbr_b200 {
 
@@ -200,10 +201,6 @@ __device__ __forceinline__ bool trace_object(const DeviceScene& S, int32_t obj, 
     }
 }
 
-__device__ __forceinline__ float safe_inv(float v) {
-    return 1.0f / (fabsf(v) > 1e-20f ? v : copysignf(1e-20f, v));
-}
-
 // The two float4s of one 32-byte row of a node (lo and hi bounds of one axis)
 // in one 256-bit load (128-byte aligned nodes).
 __device__ __forceinline__ void ld_row(const float4* p, float4& a, float4& b) {
@@ -211,28 +208,9 @@ __device__ __forceinline__ void ld_row(const float4* p, float4& a, float4& b) {
         : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
         : "l"(__cvta_generic_to_global(p)));
 }
-__device__ __forceinline__ float max3(float a, float b, float c) {
-    float r;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-__device__ __forceinline__ float min3(float a, float b, float c) {
-    float r;
-    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
 
-// A ray as the slab tests read it: 1 / d, o / d and |1 / d|.
-struct SlabRay {
-    f3 i, o, a;
-};
-__device__ __forceinline__ SlabRay slab_ray(f3 o, f3 d) {
-    SlabRay r;
-    r.i = mk(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
-    r.o = mk(o.x * r.i.x, o.y * r.i.y, o.z * r.i.z);
-    r.a = mk(fabsf(r.i.x), fabsf(r.i.y), fabsf(r.i.z));
-    return r;
-}
+__device__ __forceinline__ SlabRay slab_ray(f3 o, f3 d) { return slab_ray(o.x, o.y, o.z, d.x, d.y, d.z); }
+__device__ __forceinline__ bool slab_walks(const SlabRay& r, f3 d) { return slab_walks(r, d.x, d.y, d.z); }
 
 // Slab tests of a 4-wide node's children (t in [0, lim]): entry distances and
 // which are hit.  The boxes come as centres and half extents, so entry and
@@ -260,15 +238,7 @@ __device__ __forceinline__ Slab4 slab4(const float4* __restrict__ node, const Sl
     Slab4 s;
     s.ref[0] = rf.x; s.ref[1] = rf.y; s.ref[2] = rf.z; s.ref[3] = rf.w;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float mx = __fmaf_rn(x[k], r.i.x, -r.o.x), my = __fmaf_rn(y[k], r.i.y, -r.o.y),
-                    mz = __fmaf_rn(z[k], r.i.z, -r.o.z);
-        s.tn[k] = fmaxf(max3(__fmaf_rn(-ex[k], r.a.x, mx), __fmaf_rn(-ey[k], r.a.y, my), __fmaf_rn(-ez[k], r.a.z, mz)),
-                        0.0f);
-        const float tf = fminf(min3(__fmaf_rn(ex[k], r.a.x, mx), __fmaf_rn(ey[k], r.a.y, my),
-                                    __fmaf_rn(ez[k], r.a.z, mz)), lim);
-        s.hit[k] = s.tn[k] <= tf;
-    }
+    for (int k = 0; k < 4; ++k) s.hit[k] = slab_child(x[k], ex[k], y[k], ey[k], z[k], ez[k], r, lim, s.tn[k]);
     return s;
 }
 
@@ -383,9 +353,9 @@ __device__ __forceinline__ bool trace_scene_rt(bool ANY, bool COUNT, const Devic
             }
         }
     }
-    if (S.n_nodes == 0) return ANY ? false : best_prim != HIT_NONE;
-
     const SlabRay sr = slab_ray(o, d);
+    if (S.n_nodes == 0 || !slab_walks(sr, d)) return ANY ? false : best_prim != HIT_NONE;
+
     LocalStack st;
     st.clear();
     int32_t cur = 0;
@@ -508,7 +478,7 @@ __device__ __forceinline__ void trav_init(const DeviceScene& S, TravState& s, f3
     s.t_best = ANY ? t_limit : __int_as_float(0x7f800000);
     s.best_prim = HIT_NONE;
     s.best_key = 0xFFFFFFFFu;
-    s.cur = S.n_nodes ? 0 : TRAV_IDLE;
+    s.cur = S.n_nodes && slab_walks(s.r, d) ? 0 : TRAV_IDLE;
     s.hit = false;
     s.cache.obj = -1;
     s.cache.ok = true;

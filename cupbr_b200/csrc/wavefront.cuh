@@ -355,12 +355,15 @@ __device__ __forceinline__ void slot_path(uint32_t s, uint32_t w, uint32_t h, ui
 // Closest hits of one warp's 32 rays walked as a packet (packet_visit4):
 // every lane of the warp calls it together; a lane with valid = false takes
 // part in the walk but accepts no box.  On return s holds the lane's hit as
-// trav_run leaves it (t_best, best_prim, best_key).
+// trav_init and trav_leaf leave it (t_best, best_prim, best_key).
 __device__ __forceinline__ void packet_closest(const DeviceScene& S, f3 o, f3 d, bool valid, TravState& s,
                                                int32_t* st_ref, float* st_t, bool& overflow) {
     trav_init<false>(S, s, o, d, 0.0f);
-    // a lane past the end of the queue accepts no box (t_f <= -1 < t_n)
-    if (!valid) s.t_best = -1.0f;
+    // a lane past the end of the queue, or whose ray walks no tree, accepts no
+    // box (t_f <= -1 < t_n)
+    const bool walks = valid && s.cur == 0;
+    const float t_planes = s.t_best;
+    if (!walks) s.t_best = -1.0f;
     int sp = 0;
     int32_t cur = 0;
     uint32_t guard = 2u * S.n_nodes + 64u;
@@ -375,10 +378,11 @@ __device__ __forceinline__ void packet_closest(const DeviceScene& S, f3 o, f3 d,
             else live = packet_pop(s.t_best, st_ref, st_t, sp, cur);
         } else {
             TraceCounters tc;
-            if (valid) trav_leaf<false, false>(S, s, ~(uint32_t)cur, tc);
+            if (walks) trav_leaf<false, false>(S, s, ~(uint32_t)cur, tc);
             live = packet_pop(s.t_best, st_ref, st_t, sp, cur);
         }
     }
+    if (!walks) s.t_best = t_planes;
 }
 
 // Closest hits of a coherent queue as warp packets (packet_visit4): each
