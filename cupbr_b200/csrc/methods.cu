@@ -784,9 +784,9 @@ cudaError_t launch_gdpt_reconstruct(uint32_t w, uint32_t h, const float* base, c
     // output after an even number of launches.
     constexpr int LAUNCHES = 50 / GD_PASSES;
     static_assert(LAUNCHES * GD_PASSES == 50 && LAUNCHES % 2 == 0, "passes per launch");
-    static const cudaError_t smem =
-        cudaFuncSetAttribute(k_gdpt_opt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GD_SMEM);
-    if (smem != cudaSuccess) return smem;
+    // the opt-in belongs to the current device, so every call makes it
+    cudaError_t e = cudaFuncSetAttribute(k_gdpt_opt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GD_SMEM);
+    if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -801,7 +801,7 @@ cudaError_t launch_gdpt_reconstruct(uint32_t w, uint32_t h, const float* base, c
         const float* src = (i & 1) ? temp : out;
         float* dst = (i & 1) ? out : temp;
         const float *cgx = gx, *cgy = gy, *ctemp = temp;
-        cudaError_t e = cudaLaunchKernelEx(&cfg, k_gdpt_opt, w, h, src, cgx, cgy, ctemp, dst, i * GD_PASSES, i & 1);
+        e = cudaLaunchKernelEx(&cfg, k_gdpt_opt, w, h, src, cgx, cgy, ctemp, dst, i * GD_PASSES, i & 1);
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
