@@ -575,6 +575,7 @@ __global__ void k_rc_adam(RcNet N, uint32_t nparts, RcAdam A, float c1, float c2
     }
 }
 
+// The opt-in belongs to the current device, so every launch makes it.
 template <typename K>
 cudaError_t set_smem(K kernel, uint32_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -585,7 +586,7 @@ cudaError_t set_smem(K kernel, uint32_t bytes) {
 cudaError_t rc_infer(const RcNet& N, const __half* weights, const RcBounds& B, const float4* recs, uint32_t n,
                      float4* out, int num_sms, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    static cudaError_t attr = set_smem(k_rc_infer<false>, RC_INFER_SMEM);
+    cudaError_t attr = set_smem(k_rc_infer<false>, RC_INFER_SMEM);
     if (attr != cudaSuccess) return attr;
     const uint32_t tiles = (n + RC_TILE - 1) / RC_TILE;
     const uint32_t grid = std::min<uint32_t>(tiles, (uint32_t)num_sms * RC_INFER_BLOCKS_PER_SM);
@@ -597,7 +598,7 @@ cudaError_t rc_infer(const RcNet& N, const __half* weights, const RcBounds& B, c
 cudaError_t rc_infer_queries(const RcNet& N, const __half* weights, const RcBounds& B, const float4* recs,
                              const uint32_t* count, uint32_t capacity, float4* radiance, int num_sms, cudaStream_t st) {
     if (capacity == 0) return cudaSuccess;
-    static cudaError_t attr = set_smem(k_rc_infer<true>, RC_INFER_SMEM);
+    cudaError_t attr = set_smem(k_rc_infer<true>, RC_INFER_SMEM);
     if (attr != cudaSuccess) return attr;
     const uint32_t tiles = (capacity + RC_TILE - 1) / RC_TILE;
     const uint32_t grid = std::min<uint32_t>(tiles, (uint32_t)num_sms * RC_INFER_BLOCKS_PER_SM);
@@ -610,7 +611,7 @@ cudaError_t rc_train_step(const RcNet& N, const RcBounds& B, const float4* sampl
                           uint32_t capacity, uint32_t base, uint32_t total, uint32_t n, const RcAdam& A,
                           cudaStream_t st) {
     if (n == 0 || n % RC_TILE != 0 || n / RC_TILE > N.partial_ctas) return cudaErrorInvalidValue;
-    static cudaError_t attr = set_smem(k_rc_train, RC_TRAIN_SMEM);
+    cudaError_t attr = set_smem(k_rc_train, RC_TRAIN_SMEM);
     if (attr != cudaSuccess) return attr;
     cudaError_t e = cudaMemsetAsync(N.loss, 0, 2 * sizeof(float), st);
     if (e != cudaSuccess) return e;
