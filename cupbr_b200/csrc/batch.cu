@@ -188,13 +188,13 @@ __global__ void __launch_bounds__(256, 2) k_batch_coop(const DeviceScene* __rest
                 packet_trace<false>(S, W.rays[0], 3, nrays, &W.ctr[CTR_EFETCH + 0], &W.err[ERR_STACK],
                                     hit);
             else
-                persistent_trace<false, false, 256, false>(S, W.rays[d & 1], 3, nrays, &W.ctr[CTR_EFETCH + d], s_stack,
+                persistent_trace<false, false, 256, false>(S, W.rays[d & 1], 3, nrays, 4u, &W.ctr[CTR_EFETCH + d], s_stack,
                                                       &W.err[ERR_STACK], W.stats, hit);
             if (!grid_barrier(gb, nblocks, limit_ns)) return;
             shade_stage<false, false, false>(S, F, W, d, C);
             if (!grid_barrier(gb, nblocks, limit_ns)) return;
             const uint32_t nsh = __ldcg(&W.ctr[CTR_SHADOW + d]);
-            persistent_trace<true, false, 256, false>(S, W.shadow, 3, nsh, &W.ctr[CTR_CFETCH + d], s_stack,
+            persistent_trace<true, false, 256, false>(S, W.shadow, 3, nsh, 4u, &W.ctr[CTR_CFETCH + d], s_stack,
                                                  &W.err[ERR_STACK], W.stats, [&](uint32_t idx, const TravState& s) {
                                                      if (s.hit) return;
                                                      const float4* e = W.shadow + 3 * (size_t)idx;

@@ -138,6 +138,7 @@ struct PTBuffers {
         if ((e = alloc(&p, sizeof(uint64_t) * STAT_TOTAL)) != cudaSuccess) return e;
         ws.stats = (uint64_t*)p;
         ws.trace_blocks_per_sm = pt_occupancy_blocks();
+        ws.trace_least = 4;
         capacity = n;
         return cudaSuccess;
     }
@@ -242,6 +243,8 @@ struct cupbr_renderer_s {
     cudaStream_t stream = nullptr;
     uint64_t last_rays[2] = {0, 0};
     uint32_t batch_paths = 1u << 25;  // paths per wavefront when several frames are rendered at once
+    // Whether pipelined frames run at the same time.
+    bool overlaps() const { return pipelined && stream != nullptr && stream != cudaStreamLegacy; }
     // per-path tail kernel below this queue size (0: off); see tail()
     uint32_t tail_paths = 0;
     bool tail_set = false;
@@ -259,7 +262,7 @@ struct cupbr_renderer_s {
     // holds them up.
     PTTail tail() const {
         if (tail_set) return {tail_paths, tail_paths};
-        if (pipelined && stream != nullptr && stream != cudaStreamLegacy) return {0u, 3u << 15};
+        if (overlaps()) return {0u, 3u << 15};
         return {1u << 15, 3u << 17};
     }
     // rays of the last wavefront frame: closest-hit and shadow queue sizes
@@ -300,6 +303,16 @@ struct cupbr_renderer_s {
     size_t pipe_valid_n[PIPE_SLOTS] = {};
     cudaStream_t pipe_stream[PIPE_SLOTS] = {};
     cudaEvent_t pipe_traced[PIPE_SLOTS] = {}, pipe_folded[PIPE_SLOTS] = {};
+    // A render() call's workspace on slot k for a frame of `paths` paths.  Where
+    // frames overlap, full warps of rays (TraceShare) pay from 3 x 2^13 paths on
+    // (eight frames, us: VOLUME 64 x 64 620 against 635 with full warps, 200 x 150
+    // 719 / 690; GRADIENTDOMAIN, five paths a pixel, 64 x 64 1379 / 1457, 200 x 150
+    // 1900 / 1697).
+    Workspace pipe_workspace(uint32_t k, uint64_t paths) const {
+        Workspace w = pipe_pt[k].ws;
+        if (overlaps() && paths >= 3u << 13) w.trace_least = 32;
+        return w;
+    }
     cudaEvent_t pipe_start = nullptr;  // render_frames: the caller's stream when the call began
     cudaError_t pipe_init() {
         cudaError_t e;
@@ -845,7 +858,7 @@ static int render_gdpt(cupbr_renderer_t r, const cupbr_camera* cam, uint32_t n) 
             r->pipe_valid_n[k] = nv;
         }
         PTFrame F = make_frame(cam, r->w, r->h, r->frame, r->max_depth, false);
-        const Workspace& W = r->pipe_pt[k].ws;
+        const Workspace W = r->pipe_workspace(k, 5ull * n_int);
         CUPBR_CHECK_CUDA(cudaStreamWaitEvent(r->pipe_stream[k], r->pipe_folded[k], 0));
         CUPBR_CHECK_CUDA(gdpt_trace_frames(r->scene->g.dev, F, W, r->pipe_valid[k], r->pipe_stream[k],
                                            device_sm_count(), false));
@@ -967,7 +980,7 @@ int cupbr_renderer_render(cupbr_renderer_t r, const cupbr_camera* cam) {
                 r->pipe_next = (k + 1) % cupbr_renderer_s::PIPE_SLOTS;
                 CUPBR_CHECK_CUDA(r->pipe_init());
                 CUPBR_CHECK_CUDA(r->pipe_pt[k].ensure(r->w * r->h));
-                const Workspace& W = r->pipe_pt[k].ws;
+                const Workspace W = r->pipe_workspace(k, F.n_paths);
                 // the slot's workspace is free once its last frame was folded
                 CUPBR_CHECK_CUDA(cudaStreamWaitEvent(r->pipe_stream[k], r->pipe_folded[k], 0));
                 CUPBR_CHECK_CUDA(pt_render_frame(r->scene->g.dev, F, W, nullptr, r->pipe_stream[k], device_sm_count(),
@@ -1000,7 +1013,7 @@ int cupbr_renderer_render(cupbr_renderer_t r, const cupbr_camera* cam) {
                 r->pipe_next = (k + 1) % cupbr_renderer_s::PIPE_SLOTS;
                 CUPBR_CHECK_CUDA(r->pipe_init());
                 CUPBR_CHECK_CUDA(r->pipe_pt[k].ensure(F.n_paths));
-                const Workspace& W = r->pipe_pt[k].ws;
+                const Workspace W = r->pipe_workspace(k, F.n_paths);
                 CUPBR_CHECK_CUDA(cudaStreamWaitEvent(r->pipe_stream[k], r->pipe_folded[k], 0));
                 CUPBR_CHECK_CUDA(volume_render_frame(r->scene->g.dev, F, W, nullptr, r->pipe_stream[k],
                                                      device_sm_count(), false));

@@ -657,7 +657,7 @@ __global__ void __launch_bounds__(PT_TRACE_THREADS) k_medium_connect(DeviceScene
                                                                      double* __restrict__ lsum) {
     __shared__ __align__(8) char s_stack[LaneStack<true, PT_TRACE_THREADS>::NEAR];
     persistent_trace<true, false, PT_TRACE_THREADS>(
-        S, W.shadow, 3, W.ctr[CTR_SHADOW + depth], &W.ctr[CTR_CFETCH + depth], s_stack,
+        S, W.shadow, 3, W.ctr[CTR_SHADOW + depth], 4u, &W.ctr[CTR_CFETCH + depth], s_stack,
         &W.err[ERR_STACK], W.stats, [&](uint32_t idx, const TravState& s) {
             if (s.hit) return;
             float4* e = W.shadow + 3 * (size_t)idx;

@@ -68,8 +68,8 @@ __global__ void __launch_bounds__(PT_TRACE_THREADS, 8) k_extend(DeviceScene S, W
                                                               uint32_t min_count) {
     if (W.ctr[CTR_RAYS + depth] < min_count) return;  // cached frames: left to k_tail
     __shared__ __align__(8) char s_stack[TRACE_STACK_BYTES<PT_TRACE_THREADS>];
-    persistent_trace<false, COUNT, PT_TRACE_THREADS>(S, W.rays[depth & 1], 3, W.ctr[CTR_RAYS + depth], &W.ctr[CTR_EFETCH + depth],
-                                   s_stack, &W.err[ERR_STACK], W.stats + STAT_EXT_NODES,
+    persistent_trace<false, COUNT, PT_TRACE_THREADS>(S, W.rays[depth & 1], 3, W.ctr[CTR_RAYS + depth], W.trace_least,
+                                   &W.ctr[CTR_EFETCH + depth], s_stack, &W.err[ERR_STACK], W.stats + STAT_EXT_NODES,
                                    [&](uint32_t idx, const TravState& s) {
                                        W.hits[idx] = make_float2(s.t_best, __int_as_float(s.best_prim));
                                    });
@@ -95,8 +95,8 @@ __global__ void __launch_bounds__(PT_TRACE_THREADS) k_extend_camera(DeviceScene 
 template <bool COUNT>
 __global__ void __launch_bounds__(PT_TRACE_THREADS, 8) k_connect(DeviceScene S, Workspace W, uint32_t depth) {
     __shared__ __align__(8) char s_stack[LaneStack<true, PT_TRACE_THREADS>::NEAR];
-    persistent_trace<true, COUNT, PT_TRACE_THREADS>(S, W.shadow, 3, W.ctr[CTR_SHADOW + depth], &W.ctr[CTR_CFETCH + depth], s_stack,
-                                  &W.err[ERR_STACK], W.stats + STAT_SH_NODES,
+    persistent_trace<true, COUNT, PT_TRACE_THREADS>(S, W.shadow, 3, W.ctr[CTR_SHADOW + depth], W.trace_least,
+                                  &W.ctr[CTR_CFETCH + depth], s_stack, &W.err[ERR_STACK], W.stats + STAT_SH_NODES,
                                   [&](uint32_t idx, const TravState& s) {
                                       if (s.hit) return;
                                       const float4* e = W.shadow + 3 * (size_t)idx;

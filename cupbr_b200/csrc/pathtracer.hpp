@@ -51,6 +51,7 @@ struct Workspace {
     uint32_t* err;         // ERR_TOTAL error counters (never reset by a frame)
     uint64_t* stats;       // STAT_TOTAL traversal counters (instrumented frames only)
     int trace_blocks_per_sm;
+    uint32_t trace_least;  // rays of a queue that a traversal warp takes at least (TraceShare)
 };
 
 int pt_occupancy_blocks();

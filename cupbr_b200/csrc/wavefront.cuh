@@ -163,6 +163,11 @@ __device__ __forceinline__ uint32_t trace_chunk(uint32_t count, uint32_t end, ui
 // few lanes to each warp: its warps then diverge less, and no counter is
 // touched (its additions complete one after the other, 0.8 ns each: 4 us for
 // the warps of a grid).  Four ragged 1273 x 717 frames in flight 6.6 -> 6.0 ms.
+// Where frames overlap, other frames' warps fill the lanes that this leaves
+// empty only as warps of their own: there a warp takes `least` = 32 (pipelined
+// frames of the Cornell box, us each, 400 x 300 128 with least = 4, 99 with 32;
+// 480 x 270 120 / 96; 640 x 360 148 / 119; a scene of 40 objects of all
+// materials 99 / 101, 98 / 100, 114 / 113).
 // Packets stay with 32 rays a claim: neighbouring packets then run at the same
 // time (960 x 540 terrain 363 us, 556 with this deal).
 struct TraceShare {
@@ -235,8 +240,8 @@ struct TraceShare {
 // lanes 46.2 ms.
 template <bool ANY, bool COUNT, int THREADS, bool NC = true, typename Done>
 __device__ __forceinline__ void persistent_trace(const DeviceScene& S, const float4* __restrict__ q, uint32_t stride,
-                                                 uint32_t count, uint32_t* fetch, char* s_stack, uint32_t* err_stack,
-                                                 uint64_t* stats, Done done) {
+                                                 uint32_t count, uint32_t least, uint32_t* fetch, char* s_stack,
+                                                 uint32_t* err_stack, uint64_t* stats, Done done) {
     const unsigned full = 0xffffffffu;
     const uint32_t lane = lane_id();
     // a well-formed tree visits every node at most once per ray, and a round
@@ -247,7 +252,7 @@ __device__ __forceinline__ void persistent_trace(const DeviceScene& S, const flo
     LaneStack<ANY, THREADS> st(s_stack);
     TraceCounters tc;
     __shared__ uint32_t s_first_end;
-    TraceShare share(count, 4u, &s_first_end);
+    TraceShare share(count, least, &s_first_end);
     bool overflow = false, have = false;
     uint32_t idx = 0;
     uint32_t steps = 0;
