@@ -611,12 +611,12 @@ __device__ __forceinline__ float median4(float v0, float v1, float v2, float v3)
 
 // GD_PASSES passes of optimization_kernel (GradientDomain.cu:303-350), the
 // passes first, first + 1, .. of the reconstruction, src -> dst.  A block
-// holds a region of GD_COLS x (GD_SEGS * GD_ROWS) pixels, GD_PASSES more on
-// every side than the tile it writes: each pass leaves one more ring of
-// the region undefined.  A thread keeps GD_ROWS values of one float column
-// (column and channel: columns 3 floats apart are neighbours) and their
-// gradients in registers for all passes and reads only its left and right
-// neighbours, and the rows next to its own, from shared memory.
+// holds a region (GdRegion), GD_PASSES pixels more on every side than the tile
+// it writes: each pass leaves one more ring of the region undefined.  A
+// thread keeps ROWS values of one float column (column and channel: columns 3
+// floats apart are neighbours) and their gradients in registers for all passes
+// and reads only its left and right neighbours, and the rows next to its own,
+// from shared memory.
 // Border pixels of the image are no pass's output.  The reference copies the
 // whole of temp, its border included, over the output after every pass
 // (:392-401): pass 0 reads the border that k_gdpt_init gave the output, every
@@ -624,37 +624,49 @@ __device__ __forceinline__ float median4(float v0, float v1, float v2, float v3)
 //
 // One pass per launch pays a launch's latency for 0.5 us of arithmetic at
 // 512 x 512 (and re-reads 48 B per pixel through L2 at larger sizes); here a
-// region is read once for five.  Bound by issue (17 instructions a value and
-// pass, 1.7 times the values for the rings) and, below 512 x 512, by a block's
-// latency.  Reconstruction on a B200, one pass per launch -> this: 64 x 48 149
-// -> 118 us, 512 x 512 217 -> 132 (140 tiles on 148 SMs), 1280 x 720 535 -> 365,
-// 1920 x 1080 1300 -> 750; 3 segments of 16 rows 169 at 512 x 512, 5 of 10 143.
+// region is read once for five.  Large images take regions of 64 x 48, bound by
+// issue (17 instructions a value and pass, 1.7 times the values for the rings):
+// 512 x 512 217 us with one pass per launch -> 130 (140 tiles on 148 SMs), 1280 x
+// 720 535 -> 365, 1920 x 1080 1300 -> 750; 3 segments of 16 rows 169 at 512 x
+// 512, 5 of 10 143.  Where a block's latency is what counts, 12 rows of a
+// thread one after the other take longer than one pass per launch did (200 x
+// 150 111 us -> 123): regions of 32 x 32 with 4 rows take 48, and while they come
+// in three waves of a block per SM or fewer they stay ahead (264 x 264, one
+// wave, 50 against 126 us; 480 x 270, two, 84 / 127; 640 x 360, four, 132 / 129).
 // Launched as a chain of programmatic dependent launches: each
 // lets the next be scheduled when its own blocks start, which waits for it
 // to complete before it reads anything.
-constexpr int GD_PASSES = 5, GD_COLS = 64, GD_SEGS = 4, GD_ROWS = 12;
-constexpr int GD_TILE_W = GD_COLS - 2 * GD_PASSES, GD_TILE_H = GD_SEGS * GD_ROWS - 2 * GD_PASSES;
-constexpr int GD_ROW_FLOATS = 3 * GD_COLS, GD_THREADS = GD_ROW_FLOATS * GD_SEGS;
-constexpr int GD_PLANE = GD_SEGS * GD_ROWS * GD_ROW_FLOATS;  // floats of a region
-constexpr int GD_PAD = GD_ROW_FLOATS;                        // a row before and after it
-constexpr size_t GD_SMEM = sizeof(float) * 2 * (GD_PLANE + 2 * GD_PAD);
+constexpr int GD_PASSES = 5;
+// A region: columns, and segments of as many rows as a thread holds.
+template <int COLS_, int SEGS_, int ROWS_>
+struct GdRegion {
+    static constexpr int COLS = COLS_, SEGS = SEGS_, ROWS = ROWS_, HEIGHT = SEGS * ROWS;
+    static constexpr int TILE_W = COLS - 2 * GD_PASSES, TILE_H = HEIGHT - 2 * GD_PASSES;
+    static constexpr int ROW_FLOATS = 3 * COLS, THREADS = ROW_FLOATS * SEGS;
+    static constexpr int PLANE = HEIGHT * ROW_FLOATS;  // floats of a region
+    static constexpr int PAD = ROW_FLOATS;             // a row before and after it
+    static constexpr size_t SMEM = sizeof(float) * 2 * (PLANE + 2 * PAD);
+};
+using GdSmall = GdRegion<32, 8, 4>;
+using GdLarge = GdRegion<64, 4, 12>;
+constexpr uint64_t GD_SMALL_TILES = 3 * 148;
 
 // EDGE: the region reaches the image's border or beyond.
-template <bool EDGE>
+template <typename G, bool EDGE>
 __device__ __forceinline__ void gdpt_region(uint32_t w, uint32_t h, const float* src, const float* __restrict__ gx,
                                             const float* __restrict__ gy, const float* temp, float* dst, int first,
                                             int copy_border, float* cur, float* nxt) {
-    const int col = (int)(threadIdx.x % GD_ROW_FLOATS), row0 = (int)(threadIdx.x / GD_ROW_FLOATS) * GD_ROWS;
-    const int x = (int)blockIdx.x * GD_TILE_W - GD_PASSES + col / 3, c = col % 3;
-    const int y0 = (int)blockIdx.y * GD_TILE_H - GD_PASSES + row0;
+    const int col = (int)(threadIdx.x % G::ROW_FLOATS), row0 = (int)(threadIdx.x / G::ROW_FLOATS) * G::ROWS;
+    const int x = (int)blockIdx.x * G::TILE_W - GD_PASSES + col / 3, c = col % 3;
+    const int y0 = (int)blockIdx.y * G::TILE_H - GD_PASSES + row0;
     const int W = (int)w, H = (int)h;
     const bool in_x = !EDGE || (x >= 0 && x < W);
     const ptrdiff_t pitch = 3 * (ptrdiff_t)w, at0 = (ptrdiff_t)y0 * pitch + 3 * (ptrdiff_t)x + c;
-    float v[GD_ROWS], gxl[GD_ROWS], gxp[GD_ROWS], gyp[GD_ROWS];
+    float v[G::ROWS], gxl[G::ROWS], gxp[G::ROWS], gyp[G::ROWS];
     float gyd = 0.0f;    // gy one row below the thread's first
     uint32_t inner = 0;  // EDGE: rows whose pixel a pass computes
 #pragma unroll
-    for (int r = 0; r < GD_ROWS; ++r) {
+    for (int r = 0; r < G::ROWS; ++r) {
         const int y = y0 + r;
         const ptrdiff_t p = at0 + r * pitch;
         if (!EDGE) {
@@ -677,51 +689,52 @@ __device__ __forceinline__ void gdpt_region(uint32_t w, uint32_t h, const float*
     }
     if (!EDGE || (in_x && y0 > 0 && y0 <= H)) gyd = __ldg(&gy[at0 - pitch]);
 #pragma unroll
-    for (int r = 0; r < GD_ROWS; ++r) cur[(row0 + r) * GD_ROW_FLOATS + col] = v[r];
+    for (int r = 0; r < G::ROWS; ++r) cur[(row0 + r) * G::ROW_FLOATS + col] = v[r];
     __syncthreads();
     for (int p = 0; p < GD_PASSES; ++p) {
-        float below = cur[(row0 - 1) * GD_ROW_FLOATS + col], gb = gyd;
-        const float above = cur[(row0 + GD_ROWS) * GD_ROW_FLOATS + col];
+        float below = cur[(row0 - 1) * G::ROW_FLOATS + col], gb = gyd;
+        const float above = cur[(row0 + G::ROWS) * G::ROW_FLOATS + col];
 #pragma unroll
-        for (int r = 0; r < GD_ROWS; ++r) {
-            const float* q = cur + (row0 + r) * GD_ROW_FLOATS + col;
+        for (int r = 0; r < G::ROWS; ++r) {
+            const float* q = cur + (row0 + r) * G::ROW_FLOATS + col;
             const float old = v[r];
             const float m = median4(q[-3] + gxl[r], below + gb, q[3] - gxp[r],
-                                    (r + 1 < GD_ROWS ? v[r + 1] : above) - gyp[r]);
+                                    (r + 1 < G::ROWS ? v[r + 1] : above) - gyp[r]);
             below = old;
             gb = gyp[r];
             if (!EDGE || (inner >> r & 1u)) v[r] = m;
             else if (first + p == 0 && in_x && y0 + r >= 0 && y0 + r < H) v[r] = temp[at0 + r * pitch];
-            nxt[(row0 + r) * GD_ROW_FLOATS + col] = v[r];
+            nxt[(row0 + r) * G::ROW_FLOATS + col] = v[r];
         }
         float* t = cur;
         cur = nxt;
         nxt = t;
         __syncthreads();
     }
-    if (!in_x || col < 3 * GD_PASSES || col >= 3 * (GD_COLS - GD_PASSES)) return;
+    if (!in_x || col < 3 * GD_PASSES || col >= 3 * (G::COLS - GD_PASSES)) return;
 #pragma unroll
-    for (int r = 0; r < GD_ROWS; ++r) {
+    for (int r = 0; r < G::ROWS; ++r) {
         const int y = y0 + r, row = row0 + r;
-        if (row < GD_PASSES || row >= GD_SEGS * GD_ROWS - GD_PASSES) continue;
+        if (row < GD_PASSES || row >= G::HEIGHT - GD_PASSES) continue;
         if (!EDGE || (y >= 0 && y < H && ((inner >> r & 1u) || copy_border))) dst[at0 + r * pitch] = v[r];
     }
 }
 
-__global__ void __launch_bounds__(GD_THREADS, 1) k_gdpt_opt(uint32_t w, uint32_t h, const float* src,
+template <typename G>
+__global__ void __launch_bounds__(G::THREADS, 1) k_gdpt_opt(uint32_t w, uint32_t h, const float* src,
                                                             const float* __restrict__ gx,
                                                             const float* __restrict__ gy, const float* temp, float* dst,
                                                             int first, int copy_border) {
     extern __shared__ float s_gd[];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    float* cur = s_gd + GD_PAD;
-    float* nxt = cur + GD_PLANE + 2 * GD_PAD;
+    float* cur = s_gd + G::PAD;
+    float* nxt = cur + G::PLANE + 2 * G::PAD;
     // the region's pixels and one more below and left of it lie inside the border
-    const int x0 = (int)blockIdx.x * GD_TILE_W - GD_PASSES, y0 = (int)blockIdx.y * GD_TILE_H - GD_PASSES;
-    const bool inside = x0 > 1 && y0 > 1 && x0 + GD_COLS < (int)w && y0 + GD_SEGS * GD_ROWS < (int)h;
-    if (inside) gdpt_region<false>(w, h, src, gx, gy, temp, dst, first, copy_border, cur, nxt);
-    else gdpt_region<true>(w, h, src, gx, gy, temp, dst, first, copy_border, cur, nxt);
+    const int x0 = (int)blockIdx.x * G::TILE_W - GD_PASSES, y0 = (int)blockIdx.y * G::TILE_H - GD_PASSES;
+    const bool inside = x0 > 1 && y0 > 1 && x0 + G::COLS < (int)w && y0 + G::HEIGHT < (int)h;
+    if (inside) gdpt_region<G, false>(w, h, src, gx, gy, temp, dst, first, copy_border, cur, nxt);
+    else gdpt_region<G, true>(w, h, src, gx, gy, temp, dst, first, copy_border, cur, nxt);
 }
 
 // raytracing_kernel (RayTracer.cu:11-54): direct light from every light's
@@ -773,38 +786,49 @@ cudaError_t volume_render_frame(const DeviceScene& S, const PTFrame& F, const Wo
     return img ? pt_launch_accumulate(F, W, img, st) : cudaGetLastError();
 }
 
-cudaError_t launch_gdpt_reconstruct(uint32_t w, uint32_t h, const float* base, const float* gxf, const float* gxb,
-                                    const float* gyf, const float* gyb, float* gx, float* gy, float* temp, float* out,
-                                    cudaStream_t st) {
-    const uint32_t n = w * h;
-    if (n == 0) return cudaSuccess;
-    k_gdpt_init<<<(n + 255) / 256, 256, 0, st>>>(w, h, out, base, gxf, gxb, gyf, gyb, gx, gy);
+template <typename G>
+static cudaError_t gdpt_passes(uint32_t w, uint32_t h, const float* gx, const float* gy, float* temp, float* out,
+                               cudaStream_t st) {
     // 50 passes (GradientDomain.cu:392-401), alternating between the output and
     // temp instead of copying temp back after each: the result lands in the
     // output after an even number of launches.
     constexpr int LAUNCHES = 50 / GD_PASSES;
     static_assert(LAUNCHES * GD_PASSES == 50 && LAUNCHES % 2 == 0, "passes per launch");
+    cudaError_t e = cudaSuccess;
     // the opt-in belongs to the current device, so every call makes it
-    cudaError_t e = cudaFuncSetAttribute(k_gdpt_opt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GD_SMEM);
+    if (G::SMEM > 48 * 1024)
+        e = cudaFuncSetAttribute(k_gdpt_opt<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM);
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((w + GD_TILE_W - 1) / GD_TILE_W, (h + GD_TILE_H - 1) / GD_TILE_H);
-    cfg.blockDim = dim3(GD_THREADS);
-    cfg.dynamicSmemBytes = GD_SMEM;
+    cfg.gridDim = dim3((w + G::TILE_W - 1) / G::TILE_W, (h + G::TILE_H - 1) / G::TILE_H);
+    cfg.blockDim = dim3(G::THREADS);
+    cfg.dynamicSmemBytes = G::SMEM;
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     for (int i = 0; i < LAUNCHES; ++i) {
         const float* src = (i & 1) ? temp : out;
         float* dst = (i & 1) ? out : temp;
-        const float *cgx = gx, *cgy = gy, *ctemp = temp;
-        e = cudaLaunchKernelEx(&cfg, k_gdpt_opt, w, h, src, cgx, cgy, ctemp, dst, i * GD_PASSES, i & 1);
+        const float* ctemp = temp;
+        e = cudaLaunchKernelEx(&cfg, k_gdpt_opt<G>, w, h, src, gx, gy, ctemp, dst, i * GD_PASSES, i & 1);
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
+}
+
+cudaError_t launch_gdpt_reconstruct(uint32_t w, uint32_t h, const float* base, const float* gxf, const float* gxb,
+                                    const float* gyf, const float* gyb, float* gx, float* gy, float* temp, float* out,
+                                    cudaStream_t st) {
+    const uint32_t n = w * h;
+    if (n == 0) return cudaSuccess;
+    k_gdpt_init<<<(n + 255) / 256, 256, 0, st>>>(w, h, out, base, gxf, gxb, gyf, gyb, gx, gy);
+    const uint64_t tiles = (uint64_t)((w + GdSmall::TILE_W - 1) / GdSmall::TILE_W) *
+                           ((h + GdSmall::TILE_H - 1) / GdSmall::TILE_H);
+    return tiles <= GD_SMALL_TILES ? gdpt_passes<GdSmall>(w, h, gx, gy, temp, out, st)
+                                   : gdpt_passes<GdLarge>(w, h, gx, gy, temp, out, st);
 }
 
 cudaError_t gdpt_trace_frames(const DeviceScene& S, const PTFrame& F, const Workspace& W, void* valid_scratch,

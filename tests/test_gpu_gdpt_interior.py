@@ -1,6 +1,7 @@
 """cupbr_gdpt_reconstruct on images with tiles that lie inside the border, which
-take a kernel branch without bounds (from 114 x 82 on), beside tiles at the
-edges: bit-exact against the restatement of the 50 passes."""
+take a kernel branch without bounds, beside tiles at the edges, for both of its
+regions (tiles of 22 x 22 while 444 of them cover the image, else of 54 x 38):
+bit-exact against the restatement of the 50 passes."""
 import ctypes as C
 
 import numpy as np
@@ -14,8 +15,13 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-# the last size without such a tile and the first with one; several; ragged ones
-@pytest.mark.parametrize("w,h", [(113, 82), (114, 81), (114, 82), (162, 152), (200, 150), (331, 241)])
+# 22 x 22: tile edges, the last sizes without an interior tile and the first
+# with one, several, ragged ones; the last image of the small tiles (444) and the
+# first of the large; 54 x 38: as many tiles as fit exactly, a pixel more and
+# less, a single row and column of tiles
+@pytest.mark.parametrize("w,h", [(21, 22), (22, 22), (23, 23), (32, 32), (44, 45), (49, 50), (50, 49), (50, 50),
+                                 (113, 82), (114, 81), (114, 82), (162, 152), (200, 150), (331, 241), (264, 814),
+                                 (265, 814), (540, 456), (541, 457), (539, 455), (10001, 23), (23, 10001)])
 def test_reconstruct_interior_tiles(w, h):
     rng = np.random.default_rng(100 * w + h)
     images = [rng.random((h, w, 3), dtype=np.float32) for _ in range(2)]
