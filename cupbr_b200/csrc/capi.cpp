@@ -256,10 +256,11 @@ struct cupbr_renderer_s {
     // 960 x 540 1277 against 1376 us).  Where pipelined frames overlap, the
     // next frames' wavefronts fill the SMs that a sparse queue leaves idle: no
     // tail, and one launch up to 3 x 2^15 paths (us per frame of a long run,
-    // 256 x 256: 77 / 121, 103 / 138, 302 / 478; 362 x 362: 147 / 153,
-    // 172 / 150, 459 / 581; 512 x 512: 289 / 215, 330 / 181, 875 / 742).  They do
-    // not overlap on the legacy stream, which waits for the internal streams and
-    // holds them up.
+    // Cornell box, all materials, terrain, one launch / stages: 256 x 256 70 / 89,
+    // 86 / 95, 122 / 225; 304 x 304 95 / 97, 109 / 99, 139 / 227; 362 x 362 133 /
+    // 114, 148 / 105, 173 / 240; 512 x 512 260 / 187, 283 / 125, 315 / 282).  They
+    // do not overlap on the legacy stream, which waits for the internal streams
+    // and holds them up.
     PTTail tail() const {
         if (tail_set) return {tail_paths, tail_paths};
         if (overlaps()) return {0u, 3u << 15};
