@@ -339,7 +339,9 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch_persistent(con
 // dLoss/dImage / (frame0 + spp) (the running mean's weight of one frame).
 // One thread per path through all of its bounces (128 registers, 16 warps per
 // SM, every bounce as long as its slowest path) took 10.7 ms for 12 views of
-// three textured scenes (256 x 256 x 16, depth 5) on a B200; this 4.3.
+// three textured scenes (256 x 256 x 16, depth 5) on a B200; this 4.3.  Calls of
+// few paths do take that form (k_backward_paths): it needs one launch and no
+// buffers.
 
 // Path q of a scene (its views' frames one after the other): view, pixel,
 // frame, and the pixel's weight (0 for a view without an image gradient).
@@ -366,7 +368,32 @@ __device__ __forceinline__ f3 backward_path(const BatchBackwardSegment* __restri
     return mk(gi[3 * (size_t)tid], gi[3 * (size_t)tid + 1], gi[3 * (size_t)tid + 2]) * inv_n;
 }
 
-// Camera rays (batch_camera_slot) of the wavefront's paths p0 .. p0 + n - 1 of
+// Camera ray (batch_camera_slot) of a view's pixel and frame, for path `path`.
+__device__ __forceinline__ void backward_ray(const BatchView& v, uint32_t tid, uint32_t frame, uint32_t path,
+                                             float4& q0, float4& q1) {
+    uint32_t seed = tea4(tid, frame);
+    const uint32_t py = tid / v.width, px = tid - v.width * py;
+    const float jx = rnd(seed);
+    const float jy = rnd(seed);
+    const float rx = 2.0f * (((float)px + jx) / (float)v.width - 0.5f);
+    const float ry = 2.0f * (((float)py + jy) / (float)v.height - 0.5f);
+    const f3 wp = v.cam_pos + v.cam_z + rx * v.cam_x + ry * v.cam_y;
+    q0 = f4(v.cam_pos, __uint_as_float(path));
+    q1 = f4(normalize(wp - v.cam_pos), __uint_as_float(seed));
+}
+
+// A vertex's part of the gradient: `after` is the path's radiance from its
+// light term on.
+__device__ __forceinline__ void scatter_texel(float* __restrict__ grad_tex, const float4* __restrict__ tex,
+                                              int32_t texel, f3 g, f3 after) {
+    const f3 a = xyz(__ldg(&tex[texel]));
+    float* o = grad_tex + 3 * (size_t)texel;
+    if (a.x > 0.0f && after.x != 0.0f) atomicAdd(o, g.x * after.x / a.x);
+    if (a.y > 0.0f && after.y != 0.0f) atomicAdd(o + 1, g.y * after.y / a.y);
+    if (a.z > 0.0f && after.z != 0.0f) atomicAdd(o + 2, g.z * after.z / a.z);
+}
+
+// Camera rays of the wavefront's paths p0 .. p0 + n - 1 of
 // its scene; those of weight 0 are not traced.
 __global__ void __launch_bounds__(256) k_backward_camera(const BatchBackwardSegment* __restrict__ segs, uint32_t nseg,
                                                          const BatchView* __restrict__ views,
@@ -382,16 +409,7 @@ __global__ void __launch_bounds__(256) k_backward_camera(const BatchBackwardSegm
         R.depths[i] = 0u;
         W.radiance[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (want) {
-            const BatchView& v = views[view];
-            uint32_t seed = tea4(tid, frame);
-            const uint32_t py = tid / v.width, px = tid - v.width * py;
-            const float jx = rnd(seed);
-            const float jy = rnd(seed);
-            const float rx = 2.0f * (((float)px + jx) / (float)v.width - 0.5f);
-            const float ry = 2.0f * (((float)py + jy) / (float)v.height - 0.5f);
-            const f3 wp = v.cam_pos + v.cam_z + rx * v.cam_x + ry * v.cam_y;
-            q0 = f4(v.cam_pos, __uint_as_float(i));
-            q1 = f4(normalize(wp - v.cam_pos), __uint_as_float(seed));
+            backward_ray(views[view], tid, frame, i, q0, q1);
         }
     }
     uint32_t slot[1];
@@ -423,14 +441,81 @@ __global__ void __launch_bounds__(256) k_backward_scatter(const BatchBackwardSeg
     const f3 rad = xyz(W.radiance[i]);
     for (; depths; depths &= depths - 1u) {
         const float4 r = R.vertex[(size_t)(__ffs((int)depths) - 1) * R.stride + i];
-        const int32_t texel = __float_as_int(r.w);
-        const f3 a = xyz(__ldg(&tex[texel]));
-        const f3 after = rad - xyz(r);
-        float* o = grad_tex + 3 * (size_t)texel;
-        if (a.x > 0.0f && after.x != 0.0f) atomicAdd(o, g.x * after.x / a.x);
-        if (a.y > 0.0f && after.y != 0.0f) atomicAdd(o + 1, g.y * after.y / a.y);
-        if (a.z > 0.0f && after.z != 0.0f) atomicAdd(o + 2, g.z * after.z / a.z);
+        scatter_texel(grad_tex, tex, __float_as_int(r.w), g, rad - xyz(r));
     }
+}
+
+// The adjoint with one thread per path: each replays its path of every frame
+// and scatters its own vertices.  Work items and counter as k_batch_persistent.
+constexpr int BACKWARD_THREADS = 128;
+__global__ void __launch_bounds__(BACKWARD_THREADS, 512 / BACKWARD_THREADS)
+    k_backward_paths(const DeviceScene* __restrict__ scenes, const BatchView* __restrict__ views,
+                     const BatchItem* __restrict__ items, uint32_t n_items, uint32_t* counter, uint32_t max_depth,
+                     const float* const* __restrict__ grad_img, float* const* __restrict__ grad_tex, uint32_t* err) {
+    constexpr int WORDS = (int)(sizeof(DeviceScene) / sizeof(uint32_t));
+    __shared__ DeviceScene s_scene[BACKWARD_THREADS / 32];
+    const uint32_t lane = lane_id();
+    DeviceScene& S = s_scene[threadIdx.x >> 5];
+    uint32_t cur_scene = 0xFFFFFFFFu;
+    bool overflow = false;
+    TraceCounters tc;
+    PTFrame F{};
+    F.max_depth = max_depth;
+    F.use_rr = 0;
+    const CacheFrame C{};
+    for (;;) {
+        uint32_t it = 0;
+        if (lane == 0) it = atomicAdd(counter, 1u);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it >= n_items) break;
+        const BatchItem bi = items[it];
+        const BatchView v = views[bi.view];
+        if (v.scene != cur_scene) {
+            __syncwarp();
+            const uint32_t* src = reinterpret_cast<const uint32_t*>(scenes + v.scene);
+            uint32_t* dst = reinterpret_cast<uint32_t*>(&S);
+            for (int k = (int)lane; k < WORDS; k += 32) dst[k] = __ldg(&src[k]);
+            __syncwarp();
+            cur_scene = v.scene;
+        }
+        float* gt = grad_tex[v.scene];
+        const float* gi = grad_img[bi.view];
+        const uint32_t slot = bi.slot0 + lane;
+        if (!gt || !gi || slot >= v.width * v.height) continue;
+        const uint32_t tid = slot_pixel(slot, v.width, v.height);
+        const float inv_n = 1.0f / ((float)v.frame0 + (float)v.spp);
+        const f3 g = mk(gi[3 * (size_t)tid], gi[3 * (size_t)tid + 1], gi[3 * (size_t)tid + 2]) * inv_n;
+        if (is_zero(g)) continue;
+        for (uint32_t fr = 0; fr < v.spp; ++fr) {
+            float4 q0, q1, q2 = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+            backward_ray(v, tid, v.frame0 + fr, tid, q0, q1);
+            f3 rad = splat(0.0f);
+            int32_t rec_t[BATCH_BWD_MAX_DEPTH];
+            f3 rec_c[BATCH_BWD_MAX_DEPTH];
+            uint32_t nrec = 0;
+            for (uint32_t d = 0;; ++d) {
+                float t;
+                int32_t prim;
+                uint32_t key;
+                trace_scene_rt(false, false, S, xyz(q0), xyz(q1), 0.0f, t, prim, key, overflow, tc);
+                ShadeOut so;
+                shade_core<false, false>(S, F, C, d, q0, q1, q2, make_float2(t, __int_as_float(prim)), rad, so);
+                if (so.texel >= 0 && nrec < BATCH_BWD_MAX_DEPTH) {
+                    rec_t[nrec] = so.texel;
+                    rec_c[nrec] = rad;
+                    ++nrec;
+                }
+                if (so.sh && !trace_scene_rt(true, false, S, xyz(so.s0), xyz(so.s1), so.s0.w, t, prim, key, overflow, tc))
+                    rad += xyz(so.s2);
+                if (!so.ext) break;
+                q0 = so.e0;
+                q1 = so.e1;
+                q2 = so.e2;
+            }
+            for (uint32_t k = 0; k < nrec; ++k) scatter_texel(gt, S.tex, rec_t[k], g, rad - rec_c[k]);
+        }
+    }
+    if (overflow) atomicAdd(err, 1u);
 }
 
 }  // namespace
@@ -491,6 +576,20 @@ cudaError_t batch_launch_coop(const DeviceScene* scenes, const BatchWave* waves,
     cfg.numAttrs = 1;
     Workspace w = W;
     return cudaLaunchKernelEx(&cfg, k_batch_coop, scenes, waves, n_waves, segs, views, w, max_depth, gb, probe_ns);
+}
+
+cudaError_t batch_launch_backward_paths(const DeviceScene* scenes, const BatchView* views, const BatchItem* items,
+                                        uint32_t n_items, uint32_t* counter, uint32_t max_depth,
+                                        const float* const* grad_img, float* const* grad_tex, int num_sms,
+                                        uint32_t* err, cudaStream_t st) {
+    if (max_depth > BATCH_BWD_MAX_DEPTH) return cudaErrorInvalidValue;
+    const cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), st);
+    if (e != cudaSuccess) return e;
+    const uint32_t warps = BACKWARD_THREADS / 32;
+    const uint32_t blocks = std::min((n_items + warps - 1) / warps, (uint32_t)num_sms * (512 / BACKWARD_THREADS));
+    k_backward_paths<<<std::max(1u, blocks), BACKWARD_THREADS, 0, st>>>(scenes, views, items, n_items, counter,
+                                                                        max_depth, grad_img, grad_tex, err);
+    return cudaGetLastError();
 }
 
 cudaError_t batch_launch_backward(const DeviceScene& S, const BatchBackwardSegment* segs, uint32_t nseg,

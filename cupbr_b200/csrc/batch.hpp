@@ -97,6 +97,15 @@ int batch_persistent_occupancy(uint32_t threads, bool packet);
 
 // Deepest path the albedo-texture adjoint records (vertices per path).
 constexpr uint32_t BATCH_BWD_MAX_DEPTH = 16;
+// One thread per path (batch_launch_backward_paths) where a view has at most 2
+// frames and the paths come to at most two rounds of the 512 threads per SM it
+// keeps resident: its time goes with the frames a thread replays, while a
+// wavefront starts at 0.25 to 0.6 ms of launches and its buffers cost the first
+// call 0.4 to 0.7 ms.  Cornell box / terrain of 85,000 triangles, depth 5, us,
+// per path against wavefronts: 32 x 32 x 1 frame 126 / 250, 285 / 519; 91 x 91 x 2
+// 204 / 259, 585 / 606; 256 x 256 x 2 292 / 309, 659 / 638; 64 x 64 x 3 295 / 262,
+// 764 / 575; 384 x 384 x 2 458 / 415, 833 / 766.
+constexpr uint32_t BATCH_BWD_FEW_FRAMES = 2, BATCH_BWD_FEW_PATHS = 1024;  // paths per SM
 // Consecutive paths of one scene in the adjoint's order: view by view, frame by
 // frame; `start` is the view's first.
 struct BatchBackwardSegment {
@@ -111,6 +120,14 @@ struct TexRecord {
     uint32_t* depths;  // per path
     uint32_t stride;   // paths of a wavefront
 };
+// The adjoint below for all textured scenes of a launch (grad_tex per scene,
+// null for the others), one thread per path over the work items of the
+// persistent kernel: one launch, no buffers.  `counter` is reset first; `err`
+// counts traversal stack overflows.
+cudaError_t batch_launch_backward_paths(const DeviceScene* scenes, const BatchView* views, const BatchItem* items,
+                                        uint32_t n_items, uint32_t* counter, uint32_t max_depth,
+                                        const float* const* grad_img, float* const* grad_tex, int num_sms,
+                                        uint32_t* err, cudaStream_t st);
 // Adjoint of a launch's frames with respect to the albedo texture of scene S:
 // grad_tex (tex_w * tex_h RGB floats) += the derivative of the sum over the
 // scene's views and pixels of grad_img[view][pixel] . image[pixel]

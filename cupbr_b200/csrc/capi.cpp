@@ -1700,57 +1700,79 @@ struct cupbr_batch_s {
     // albedo-texture adjoint: per scene its gradient (tex_w * tex_h RGB,
     // null for untextured scenes), and the device pointer tables of a call
     std::vector<float*> tex_grad;
-    const float** dgrad_img = nullptr;
-    // the adjoint's own wavefront (a launch on another stream may use pt)
-    PTBuffers bwd_pt;
+    // its device tables: image gradients per view, texture gradients per scene,
+    // segments per view, the work item counter, error counters
+    char* bwd_tables = nullptr;
+    std::vector<char> bwd_host;
+    size_t bwd_off_tex() const { return sizeof(float*) * views.size(); }
+    size_t bwd_off_segs() const { return (bwd_off_tex() + sizeof(float*) * scenes.size() + 15) & ~(size_t)15; }
+    size_t bwd_off_counter() const { return bwd_off_segs() + sizeof(BatchBackwardSegment) * views.size(); }
+    uint32_t* bwd_counter() const { return reinterpret_cast<uint32_t*>(bwd_tables + bwd_off_counter()); }
+    uint32_t* bwd_err() const { return bwd_counter() + 1; }
+    // the adjoint's own wavefront (a launch on another stream may use pt), in one allocation
+    char* bwd_slab = nullptr;
+    Workspace bwd_ws{};
     TexRecord bwd_rec{};
-    BatchBackwardSegment* bwd_segs = nullptr;
-    uint32_t bwd_segs_n = 0;
-    uint32_t bwd_paths = 1u << 22;  // paths of a wavefront at most
     ~cupbr_batch_s() {
         release_graph();
         free_tables();
         for (float* g : tex_grad) if (g) cudaFree(g);
-        if (dgrad_img) cudaFree(dgrad_img);
-        release_record();
-        if (bwd_segs) cudaFree(bwd_segs);
+        if (bwd_tables) cudaFree(bwd_tables);
+        if (bwd_slab) cudaFree(bwd_slab);
         if (cap) cudaStreamDestroy(cap);
     }
-    void release_record() {
-        if (bwd_rec.vertex) cudaFree(bwd_rec.vertex);
-        if (bwd_rec.depths) cudaFree(bwd_rec.depths);
-        bwd_rec = TexRecord{};
+    // Cuts the wavefront of n paths out of `slab` (null: only adds up); its bytes.
+    size_t backward_layout(char* slab, uint32_t n, Workspace& w, TexRecord& rec) const {
+        size_t at = 0;
+        auto take = [&](auto*& p, size_t bytes) {
+            p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(slab ? slab + at : nullptr);
+            at += (bytes + 255) & ~(size_t)255;
+        };
+        take(w.radiance, sizeof(float4) * (size_t)n);
+        take(w.rays[0], sizeof(float4) * 3 * (size_t)n);
+        take(w.rays[1], sizeof(float4) * 3 * (size_t)n);
+        take(w.hits, sizeof(float2) * (size_t)n);
+        take(w.shadow, sizeof(float4) * 3 * (size_t)n);
+        take(w.ctr, sizeof(uint32_t) * CTR_TOTAL);
+        take(w.stats, sizeof(uint64_t) * STAT_TOTAL);
+        take(rec.vertex, sizeof(float4) * (size_t)n * max_depth);
+        take(rec.depths, sizeof(uint32_t) * (size_t)n);
+        rec.stride = n;
+        return at;
     }
     // Buffers of the adjoint for at most `paths` paths of a scene: wavefronts
-    // of 2^22 (1 GB at depth 5; 2^20 took 13 % longer for 1.7M paths a scene), halved
-    // while the device has no room for them.
-    cudaError_t backward_buffers(uint64_t paths, uint32_t n_segs) {
-        cudaError_t e = cudaSuccess;
-        if (bwd_segs_n < n_segs) {
-            if (bwd_segs) cudaFree(bwd_segs);
-            bwd_segs = nullptr;
-            bwd_segs_n = 0;
-            if ((e = dev_alloc(&bwd_segs, sizeof(BatchBackwardSegment) * n_segs)) != cudaSuccess) return e;
-            bwd_segs_n = n_segs;
-        }
-        const uint32_t want = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(paths, 1), bwd_paths);
+    // of 2^22 (1 GB at depth 5; 2^20 took 13 % longer for 1.7M paths a scene),
+    // halved while the device has no room for them and made larger once it
+    // has.  cudaErrorMemoryAllocation: no room for 2^10 paths.
+    cudaError_t backward_buffers(uint64_t paths) {
+        const uint32_t want = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(paths, 1), 1u << 22);
         if (bwd_rec.stride >= want) return cudaSuccess;
+        Workspace w{};
+        TexRecord rec{};
+        if (bwd_slab) {
+            size_t room = 0, total = 0;
+            cudaError_t e = cudaMemGetInfo(&room, &total);
+            if (e != cudaSuccess) return e;
+            if (room + backward_layout(nullptr, bwd_rec.stride, w, rec) < backward_layout(nullptr, want, w, rec))
+                return cudaSuccess;
+            cudaFree(bwd_slab);
+            bwd_slab = nullptr;
+        }
+        bwd_rec = TexRecord{};
         for (uint32_t n = want;; n = (n + 1) / 2) {
-            release_record();
-            e = bwd_pt.ensure(n);
-            if (e == cudaSuccess) e = dev_alloc(&bwd_rec.vertex, sizeof(float4) * (size_t)n * max_depth);
-            if (e == cudaSuccess) e = dev_alloc(&bwd_rec.depths, sizeof(uint32_t) * (size_t)n);
+            cudaError_t e = dev_alloc(&bwd_slab, backward_layout(nullptr, n, w, rec));
             if (e == cudaSuccess) {
-                bwd_rec.stride = n;
+                backward_layout(bwd_slab, n, w, rec);
+                w.err = bwd_err();
+                w.trace_blocks_per_sm = pt_occupancy_blocks();
+                w.trace_least = 4;
+                bwd_ws = w;
+                bwd_rec = rec;
                 return cudaSuccess;
             }
-            if (e != cudaErrorMemoryAllocation || n <= (1u << 14)) {
-                release_record();
-                return e;
-            }
+            bwd_slab = nullptr;
             (void)cudaGetLastError();
-            bwd_pt.release();
-            bwd_paths = (n + 1) / 2;
+            if (e != cudaErrorMemoryAllocation || n <= (1u << 10)) return e;
         }
     }
     void release_graph() {
@@ -2027,9 +2049,9 @@ int cupbr_batch_get_error_count(cupbr_batch_t b, uint32_t* out) {
         CUPBR_CHECK_CUDA(cudaMemcpy(e, b->pt.ws.err, sizeof e, cudaMemcpyDeviceToHost));
         for (uint32_t k = 0; k < ERR_TOTAL; ++k) *out += e[k];
     }
-    if (b->bwd_pt.ws.err) {
+    if (b->bwd_tables) {
         uint32_t e[ERR_TOTAL];
-        CUPBR_CHECK_CUDA(cudaMemcpy(e, b->bwd_pt.ws.err, sizeof e, cudaMemcpyDeviceToHost));
+        CUPBR_CHECK_CUDA(cudaMemcpy(e, b->bwd_err(), sizeof e, cudaMemcpyDeviceToHost));
         for (uint32_t k = 0; k < ERR_TOTAL; ++k) *out += e[k];
     }
     if (b->dbar) {
@@ -2067,39 +2089,62 @@ int cupbr_batch_backward(cupbr_batch_t b, const uint64_t* device_grad_images, in
         CUPBR_CHECK_CUDA(cudaStreamSynchronize(st));
         CUPBR_CHECK_CUDA(b->build(b->views));
     }
-    if (!b->dgrad_img) CUPBR_CHECK_CUDA(dev_alloc(&b->dgrad_img, sizeof(float*) * nv));
-    std::vector<const float*> gi(nv);
-    for (size_t i = 0; i < nv; ++i) gi[i] = reinterpret_cast<const float*>(device_grad_images[i]);
-    CUPBR_CHECK_CUDA(cudaMemcpyAsync(b->dgrad_img, gi.data(), sizeof(float*) * nv, cudaMemcpyHostToDevice, st));
+    const size_t table_bytes = b->bwd_off_counter();
+    if (!b->bwd_tables) {
+        const size_t counters = sizeof(uint32_t) * (1 + ERR_TOTAL);
+        CUPBR_CHECK_CUDA(dev_alloc(&b->bwd_tables, table_bytes + counters));
+        CUPBR_CHECK_CUDA(cudaMemsetAsync(b->bwd_tables + table_bytes, 0, counters, st));
+    }
     if (b->dirty) {
         CUPBR_CHECK_CUDA(cudaMemcpyAsync(b->dviews, b->views.data(), sizeof(BatchView) * nv, cudaMemcpyHostToDevice, st));
         b->dirty = false;
     }
-    // per scene the paths of its views, and wavefronts to replay them in
-    std::vector<BatchBackwardSegment> segs;
+    // per scene the paths of its views
+    b->bwd_host.resize(table_bytes);
+    char* host = b->bwd_host.data();
+    std::memcpy(host, device_grad_images, sizeof(float*) * nv);
+    std::memcpy(host + b->bwd_off_tex(), b->tex_grad.data(), sizeof(float*) * ns);
+    auto* segs = reinterpret_cast<BatchBackwardSegment*>(host + b->bwd_off_segs());
     std::vector<uint32_t> seg0(ns + 1, 0);
     std::vector<uint64_t> paths(ns, 0);
-    uint64_t most = 0;
-    for (size_t i = 0; i < ns; ++i) {
-        seg0[i] = (uint32_t)segs.size();
+    uint64_t most = 0, all = 0;
+    uint32_t spp = 0;
+    for (size_t i = 0, k = 0; i < ns; ++i) {
         for (size_t v = 0; v < nv; ++v) {
             if (b->view_scene[v] != i) continue;
-            segs.push_back(BatchBackwardSegment{paths[i], (uint32_t)v, 0u});
+            segs[k++] = BatchBackwardSegment{paths[i], (uint32_t)v, 0u};
             paths[i] += (uint64_t)b->views[v].width * b->views[v].height * b->views[v].spp;
+            if (b->tex_grad[i]) spp = std::max(spp, b->views[v].spp);
         }
-        if (b->tex_grad[i]) most = std::max(most, paths[i]);
+        seg0[i + 1] = (uint32_t)k;
+        if (b->tex_grad[i]) {
+            most = std::max(most, paths[i]);
+            all += paths[i];
+        }
     }
-    seg0[ns] = (uint32_t)segs.size();
-    CUPBR_CHECK_CUDA(b->backward_buffers(most, (uint32_t)segs.size()));
-    CUPBR_CHECK_CUDA(cudaMemcpyAsync(b->bwd_segs, segs.data(), sizeof(BatchBackwardSegment) * segs.size(),
-                                     cudaMemcpyHostToDevice, st));
-    for (size_t i = 0; i < ns; ++i) {
-        if (!b->tex_grad[i]) continue;
-        CUPBR_CHECK_CUDA(batch_launch_backward(b->scenes[i]->g.dev, b->bwd_segs + seg0[i], seg0[i + 1] - seg0[i],
-                                               b->dviews, paths[i], b->bwd_pt.ws, b->bwd_rec, b->max_depth,
-                                               b->dgrad_img, b->tex_grad[i], device_sm_count(), st));
+    CUPBR_CHECK_CUDA(cudaMemcpyAsync(b->bwd_tables, host, table_bytes, cudaMemcpyHostToDevice, st));
+    auto* grad_img = reinterpret_cast<const float* const*>(b->bwd_tables);
+    auto* grad_tex = reinterpret_cast<float* const*>(b->bwd_tables + b->bwd_off_tex());
+    auto* dsegs = reinterpret_cast<const BatchBackwardSegment*>(b->bwd_tables + b->bwd_off_segs());
+    bool waves = spp > BATCH_BWD_FEW_FRAMES || all > (uint64_t)BATCH_BWD_FEW_PATHS * device_sm_count();
+    if (waves) {
+        const cudaError_t e = b->backward_buffers(most);
+        waves = e != cudaErrorMemoryAllocation;  // no room: one thread per path needs none
+        if (waves) CUPBR_CHECK_CUDA(e);
     }
-    // the host tables above are pageable: the copies are done when the calls return
+    if (waves) {
+        for (size_t i = 0; i < ns; ++i) {
+            if (!b->tex_grad[i]) continue;
+            CUPBR_CHECK_CUDA(batch_launch_backward(b->scenes[i]->g.dev, dsegs + seg0[i], seg0[i + 1] - seg0[i], b->dviews,
+                                                   paths[i], b->bwd_ws, b->bwd_rec, b->max_depth, grad_img,
+                                                   b->tex_grad[i], device_sm_count(), st));
+        }
+    } else {
+        CUPBR_CHECK_CUDA(batch_launch_backward_paths(b->dscenes, b->dviews, b->ditems, b->n_items, b->bwd_counter(),
+                                                     b->max_depth, grad_img, grad_tex, device_sm_count(),
+                                                     b->bwd_err() + ERR_STACK, st));
+    }
+    // the host table above is pageable: the copy is done when the call returns
     CUPBR_CHECK_CUDA(cudaStreamSynchronize(st));
     return CUPBR_OK;
 }

@@ -584,7 +584,9 @@ int cupbr_batch_autotune(cupbr_batch_t b, void* stream, float* best_ms);
  * device_grad_images: one device pointer per view (width*height RGB floats
  * of dLoss/dImage, or 0 to skip the view).  Every path of the frames the
  * launch traced (frame0 .. frame0 + spp - 1 of each view) is re-traced from
- * its seed by the persistent kernel's work items; at each textured Lambert
+ * its seed, in wavefronts whose buffers the batch allocates in the first such
+ * call and keeps (at most 2^22 paths; fewer, or none, where memory is short),
+ * or by one thread per path where there are few; at each textured Lambert
  * vertex the derivative of the path's radiance with respect to that
  * vertex's texel -- (path radiance - radiance gathered before the vertex's
  * light term) / albedo per channel -- is scattered with weight
