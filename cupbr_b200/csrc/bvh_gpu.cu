@@ -919,6 +919,25 @@ struct Stats {
     uint32_t max_depth;
 };
 
+// Centre and half extent of [lo, hi], rounded outwards: the box they span
+// holds [lo, hi], with 2^-20 of the extent to spare for the traversal's
+// arithmetic on them.  A missing child (inverted bounds) gets half extent
+// -inf, which slab_child turns down for every ray that walks a tree
+// (slab_walks); a bound too large to carry its opposite's position gets a box
+// around the origin.
+__device__ __forceinline__ void slab_axis(float lo, float hi, bool empty, float& c, float& h) {
+    if (empty) {
+        c = 0.0f;
+        h = -INFINITY;
+        return;
+    }
+    const float m = fmaxf(fabsf(lo), fabsf(hi));
+    c = m < 1e15f ? 0.5f * lo + 0.5f * hi : 0.0f;
+    h = m < 1e15f ? fmaxf(__fsub_ru(hi, c), __fsub_ru(c, lo)) : m;
+    h = __fmul_ru(h, 1.0f + 1.0f / 1048576.0f);
+}
+
+// The builder's nodes (child bounds) to `out`, the traversal's to out + n4 nodes.
 __global__ void k_write_nodes(const W4* __restrict__ w4, uint32_t n4, const uint32_t* __restrict__ pos,
                               const DNode* __restrict__ nodes, float* __restrict__ out, float root_area,
                               float trav_cost, Stats* __restrict__ st) {
@@ -926,6 +945,7 @@ __global__ void k_write_nodes(const W4* __restrict__ w4, uint32_t n4, const uint
     if (v >= n4) return;
     const W4 w = w4[v];
     float* o = out + (size_t)pos[v] * (4 * BVH_NODE_F4);
+    float* q = o + (size_t)n4 * (4 * BVH_NODE_F4);
     uint32_t leaves = 0;
     double sah = 0.0;
     for (int k = 0; k < 4; ++k) {
@@ -948,32 +968,15 @@ __global__ void k_write_nodes(const W4* __restrict__ w4, uint32_t n4, const uint
         o[12 + k] = hi[1];
         o[16 + k] = lo[2];
         o[20 + k] = hi[2];
-        o[24 + k] = __int_as_float(ref);
-        o[28 + k] = 0.0f;
+        for (int a = 0; a < 3; ++a) slab_axis(lo[a], hi[a], ref == BVH_EMPTY, q[8 * a + k], q[8 * a + 4 + k]);
+        o[24 + k] = q[24 + k] = __int_as_float(ref);
+        o[28 + k] = q[28 + k] = 0.0f;
     }
     const DNode s = nodes[w.src];
     if (root_area > 0) sah += (double)(trav_cost * harea(s.lo, s.hi) / root_area);
     atomicAdd(&st->leaves, (unsigned long long)leaves);
     atomicAdd(&st->sah, sah);
     atomicMax(&st->max_depth, (uint32_t)w.depth + 1);
-}
-
-// Centre and half extent of [lo, hi], rounded outwards: the box they span
-// holds [lo, hi], with 2^-20 of the extent to spare for the traversal's
-// arithmetic on them.  A missing child (inverted bounds) gets half extent
-// -inf, which slab_child turns down for every ray that walks a tree
-// (slab_walks); a bound too large to carry its opposite's position gets a box
-// around the origin.
-__device__ __forceinline__ void slab_axis(float lo, float hi, bool empty, float& c, float& h) {
-    if (empty) {
-        c = 0.0f;
-        h = -INFINITY;
-        return;
-    }
-    const float m = fmaxf(fabsf(lo), fabsf(hi));
-    c = m < 1e15f ? 0.5f * lo + 0.5f * hi : 0.0f;
-    h = m < 1e15f ? fmaxf(__fsub_ru(hi, c), __fsub_ru(c, lo)) : m;
-    h = __fmul_ru(h, 1.0f + 1.0f / 1048576.0f);
 }
 
 __global__ void k_slab_nodes(const float4* __restrict__ in, uint32_t n, float4* __restrict__ out) {
@@ -1010,9 +1013,23 @@ inline uint32_t blocks_for(uint64_t n, uint32_t t) { return (uint32_t)std::max<u
 
 }  // namespace
 
-cudaError_t launch_slab_nodes(const float4* bounds, uint32_t n, float4* out, cudaStream_t st) {
-    if (n) k_slab_nodes<<<blocks_for(n, 128), 128, 0, st>>>(bounds, n, out);
-    return cudaGetLastError();
+cudaError_t upload_nodes(const FlatBvh& bvh, float4** d_nodes, uint32_t* n_nodes, cudaStream_t st) {
+    const uint32_t n = (uint32_t)(bvh.nodes.size() / (4 * BVH_NODE_F4));
+    float4* dn = nullptr;
+    cudaError_t e = dev_alloc(&dn, 2 * (size_t)n * BVH_NODE_BYTES);
+    if (e != cudaSuccess) return e;
+    e = cudaMemcpyAsync(dn, bvh.nodes.data(), (size_t)n * BVH_NODE_BYTES, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) {
+        k_slab_nodes<<<blocks_for(n, 128), 128, 0, st>>>(dn, n, dn + (size_t)n * BVH_NODE_F4);
+        e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) {
+        cudaFree(dn);
+        return e;
+    }
+    *d_nodes = dn;
+    *n_nodes = n;
+    return cudaSuccess;
 }
 
 bool build_bvh_device(const std::vector<PrimBox>* boxes, int ntypes, const uint32_t* slot_offset,
@@ -1032,12 +1049,11 @@ bool build_bvh_device(const std::vector<PrimBox>* boxes, int ntypes, const uint3
     if (total == 0) {
         // empty scene: the host builder's single node of empty children
         build_bvh(boxes, ntypes, slot_offset, p, perm, out);
-        float4* dn = nullptr;
-        if ((e = dev_alloc(&dn, out.nodes.size() * sizeof(float))) != cudaSuccess) return fail("cudaMalloc");
-        e = cudaMemcpy(dn, out.nodes.data(), out.nodes.size() * sizeof(float), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) { cudaFree(dn); return fail("cudaMemcpy"); }
-        *d_nodes = dn;
-        *n_nodes = (uint32_t)(out.nodes.size() / (4 * BVH_NODE_F4));
+        if ((e = upload_nodes(out, d_nodes, n_nodes, st)) != cudaSuccess) return fail("upload");
+        if ((e = cudaStreamSynchronize(st)) != cudaSuccess) {
+            cudaFree(*d_nodes);
+            return fail("upload");
+        }
         return true;
     }
     Scratch S;
@@ -1341,7 +1357,7 @@ bool build_bvh_device(const std::vector<PrimBox>* boxes, int ntypes, const uint3
         k_layout_down<<<blocks_for(cnt, 128), 128, 0, st>>>(lvl + b, cnt, w4, size, pos);
     }
     float* dn = nullptr;
-    if ((e = dev_alloc(&dn, (size_t)n4 * BVH_NODE_BYTES)) != cudaSuccess) return fail("cudaMalloc");
+    if ((e = dev_alloc(&dn, 2 * (size_t)n4 * BVH_NODE_BYTES)) != cudaSuccess) return fail("cudaMalloc");
     k_write_nodes<<<blocks_for(n4, 128), 128, 0, st>>>(w4, n4, pos, nodes, dn, root_area, p.trav_cost, dstat);
     Stats hs{};
     out.nodes.assign(4 * BVH_NODE_F4, 0.0f);

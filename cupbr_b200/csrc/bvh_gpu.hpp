@@ -22,16 +22,20 @@ namespace cupbr_b200 {
 
 // boxes[t]: primitive boxes of type t (as for build_bvh); perm[t] receives
 // the leaf order; *d_nodes receives a cudaMalloc'd array of *n_nodes 4-wide
-// nodes (the caller frees it); out.stats as build_bvh sets them, out.nodes
+// nodes and, behind them, the same nodes as the traversal reads them (the
+// caller frees it): same order and child references, per axis the four
+// children's centres and half extents instead of their bounds.  Both come from
+// one allocation and one kernel: an allocation and a launch of their own for the
+// second form took 20 us of a 20-primitive scene's commit.  out.stats as
+// build_bvh sets them, out.nodes
 // a host copy of the root node only.  Work is ordered on `st`; the call
 // returns after it has finished.
 bool build_bvh_device(const std::vector<PrimBox>* boxes, int ntypes, const uint32_t* slot_offset,
                       const BvhBuildParams& p, std::vector<uint32_t>* perm, FlatBvh& out, float4** d_nodes,
                       uint32_t* n_nodes, cudaStream_t st, std::string& err);
 
-// The traversal's node array from the builder's (bvh_build.hpp), same order
-// and child references: per axis the four children's centres and half
-// extents instead of their bounds.
-cudaError_t launch_slab_nodes(const float4* bounds, uint32_t n, float4* out, cudaStream_t st);
+// The same array for a tree built on the host; returns before `st` has made the
+// traversal's half.
+cudaError_t upload_nodes(const FlatBvh& bvh, float4** d_nodes, uint32_t* n_nodes, cudaStream_t st);
 
 }  // namespace cupbr_b200

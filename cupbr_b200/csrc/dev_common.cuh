@@ -127,7 +127,7 @@ struct DLight {  // Light.h:20-71 with the area light's normal and area precompu
 };
 
 struct DeviceScene {
-    const float4* __restrict__ nodes;     // BVH_NODE_F4 per node: children's box centres and half extents (launch_slab_nodes)
+    const float4* __restrict__ nodes;     // BVH_NODE_F4 per node: children's box centres and half extents (slab.hpp)
     const float4* __restrict__ tris;      // 3 per triangle slot: (v1, key), (v2 - v1, obj), (v3 - v1, 0)
     const float4* __restrict__ tri_n;     // 1 per triangle slot: normal.xyz
     const float4* __restrict__ spheres;   // 2 per sphere slot: (center, key), (radius, radius^2, obj, 0)

@@ -61,26 +61,6 @@ struct HostArray {
     bool empty() const { return n == 0; }
 };
 
-// The traversal's form of the committed tree's nodes (dev.nodes).
-bool make_slab_nodes(GpuScene& g, std::string& err) {
-    g.dev.nodes = nullptr;
-    if (g.dev.n_nodes == 0) return true;
-    const size_t bytes = (size_t)g.dev.n_nodes * BVH_NODE_BYTES;
-    void* p = nullptr;
-    cudaError_t e = dev_alloc(&p, bytes);
-    if (e == cudaSuccess) {
-        g.buffers.push_back(p);
-        g.device_bytes += bytes;
-        e = launch_slab_nodes(g.bounds, g.dev.n_nodes, static_cast<float4*>(p), 0);
-    }
-    if (e != cudaSuccess) {
-        err = std::string("traversal nodes: ") + cudaGetErrorString(e);
-        return false;
-    }
-    g.dev.nodes = static_cast<const float4*>(p);
-    return true;
-}
-
 template <typename Cont, typename T>
 bool upload(GpuScene& g, const Cont& v, const T*& out, std::string& err) {
     if (v.empty()) { out = nullptr; return true; }
@@ -286,18 +266,27 @@ bool commit_scene(GpuScene& g, const BvhBuildParams& params, std::string& err) {
 
     uint32_t offs[3] = {0u, (uint32_t)nT, (uint32_t)(nT + nS)};
     std::vector<uint32_t> perm[3];
-    float4* dev_nodes = nullptr;  // device build: the node array is already on the GPU
+    float4* dev_nodes = nullptr;
     uint32_t dev_n_nodes = 0;
     const auto t_bvh = std::chrono::steady_clock::now();
     g.bvh_device = params.device;
     if (params.device) {
         if (!build_bvh_device(boxes, 3, offs, params, perm, g.bvh, &dev_nodes, &dev_n_nodes, 0, err)) return false;
-        g.buffers.push_back(dev_nodes);
-        g.device_bytes += (uint64_t)dev_n_nodes * BVH_NODE_BYTES;
     } else {
         build_bvh(boxes, 3, offs, params, perm, g.bvh);
     }
     g.bvh_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_bvh).count();
+    if (!dev_nodes) {
+        // the copies of the tables below wait for it; an empty scene has none
+        cudaError_t e = upload_nodes(g.bvh, &dev_nodes, &dev_n_nodes, 0);
+        if (e == cudaSuccess && nobj == 0) e = cudaStreamSynchronize(0);
+        if (e != cudaSuccess) {
+            err = std::string("BVH nodes: ") + cudaGetErrorString(e);
+            return false;
+        }
+    }
+    g.buffers.push_back(dev_nodes);
+    g.device_bytes += 2 * (uint64_t)dev_n_nodes * BVH_NODE_BYTES;
     // A 4-wide traversal pushes at most 3 entries per level of the path it is
     // on, and the culled entries are popped first, so in practice the stack
     // stays far below 3 x depth; an overflow is still counted on the device
@@ -398,17 +387,9 @@ bool commit_scene(GpuScene& g, const BvhBuildParams& params, std::string& err) {
 
     DeviceScene& D = g.dev;
     const F4* p;
-    if (dev_nodes) {
-        g.bounds = dev_nodes;
-        D.n_nodes = dev_n_nodes;
-    } else {
-        std::vector<F4> nodes(g.bvh.nodes.size() / 4);
-        std::memcpy(nodes.data(), g.bvh.nodes.data(), g.bvh.nodes.size() * sizeof(float));
-        if (!upload(g, nodes, p, err)) return false;
-        g.bounds = reinterpret_cast<const float4*>(p);
-        D.n_nodes = (uint32_t)(nodes.size() / BVH_NODE_F4);  // nodes, not float4s
-    }
-    if (!make_slab_nodes(g, err)) return false;
+    g.bounds = dev_nodes;
+    D.nodes = dev_nodes + (size_t)dev_n_nodes * BVH_NODE_F4;
+    D.n_nodes = dev_n_nodes;
     if (!upload(g, tris, p, err)) return false;
     D.tris = reinterpret_cast<const float4*>(p);
     if (!upload(g, trin, p, err)) return false;
