@@ -515,11 +515,11 @@ __device__ __forceinline__ bool trav_accept(const DeviceScene& S, TravState& s, 
 template <bool ANY, bool COUNT>
 __device__ __forceinline__ bool trav_leaf(const DeviceScene& S, TravState& s, uint32_t v, TraceCounters& ctr) {
     const uint32_t start = v >> 3, cnt = (v & 7u) + 1u;
-    if (COUNT) ctr.tris += cnt;
     float t;
     if (start < S.sphere_base) {
         const float4* p = S.tris + 3 * (size_t)start;
         for (uint32_t k = 0; k < cnt; ++k, p += 3) {
+            if (COUNT) ctr.tris++;
             const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
             if (isect_tri(a, b, c, s.o, s.d, t) &&
                 trav_accept<ANY>(S, s, t, __float_as_uint(a.w), __float_as_int(b.w), prim_ref(0, start + k)))
@@ -529,6 +529,7 @@ __device__ __forceinline__ bool trav_leaf(const DeviceScene& S, TravState& s, ui
         const uint32_t first = start - S.sphere_base;
         const float4* p = S.spheres + 2 * (size_t)first;
         for (uint32_t k = 0; k < cnt; ++k, p += 2) {
+            if (COUNT) ctr.tris++;
             const float4 a = __ldg(p), b = __ldg(p + 1);
             if (isect_sphere(a, b, s.o, s.d, t) &&
                 trav_accept<ANY>(S, s, t, __float_as_uint(a.w), __float_as_int(b.z), prim_ref(1, first + k)))
@@ -538,6 +539,7 @@ __device__ __forceinline__ bool trav_leaf(const DeviceScene& S, TravState& s, ui
         const uint32_t first = start - S.quad_base;
         const float4* p = S.quads + 4 * (size_t)first;
         for (uint32_t k = 0; k < cnt; ++k, p += 4) {
+            if (COUNT) ctr.tris++;
             const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3);
             // a quad's object box is infinite
             if (isect_quad(a, b, c, d, s.o, s.d, t) &&
