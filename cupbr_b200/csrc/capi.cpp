@@ -1419,9 +1419,13 @@ int cupbr_postprocessor_destroy(cupbr_postprocessor_t p) {
 int cupbr_postprocessor_register_image(cupbr_postprocessor_t p, const float* hdr, uint32_t w, uint32_t h) {
     if (!p || !hdr) return fail(CUPBR_ERR_ARG, "null argument");
     if (w < 2 || h < 2) return fail(CUPBR_ERR_ARG, "bloom needs an image of at least 2x2 pixels");
-    if (p->out) cudaFree(p->out);
-    p->out = nullptr;
-    CUPBR_CHECK_CUDA(dev_alloc(&p->out, sizeof(float) * 3 * (size_t)w * h));
+    // an image of the same size keeps the output buffer
+    if (!p->out || (uint64_t)p->w * p->h != (uint64_t)w * h) {
+        if (p->out) cudaFree(p->out);
+        p->out = nullptr;
+        p->hdr = nullptr;
+        CUPBR_CHECK_CUDA(dev_alloc(&p->out, sizeof(float) * 3 * (size_t)w * h));
+    }
     p->hdr = hdr;
     p->w = w;
     p->h = h;
