@@ -13,7 +13,7 @@ render_frames, which folds several frames into one wavefront.
 Metric: Mpaths/s (paths = pixel samples).  `value` is device time of the K
 frames with the scene resident in HBM; `e2e` times K single-frame steps
 through the public API, each with the tone-mapped RGBA8 frame read back to
-pinned host memory.  The 1M-triangle inputs (222 MB resident) exceed the
+pinned host memory.  The 1M-triangle inputs (265 MB resident) exceed the
 126 MB L2; the Cornell box does not (stated in config.l2).
 `reference_cuda` is the reference's own CUDA path (oracle/_ref/libref_cuda.so,
 built for sm_100a with -use_fast_math) timed live on the same GPU.
@@ -53,7 +53,7 @@ SCENES = {
         metric="Mpaths/s (NEE path tracing, 1 spp per step, 1M-triangle scene)",
         workload="1M-triangle heightfield + 200 icospheres (2,024,000 tris), 1920x1080, depth 8, "
                  "Lambert/GGX/dielectric, 2048x1024 sky, 1 spp per step",
-        l2="inputs larger than L2 (scene 222 MB resident)", ref_res=(960, 540), ref_frames=1),
+        l2="inputs larger than L2 (scene 265 MB resident)", ref_res=(960, 540), ref_frames=1),
     "medium": dict(
         W=512, H=512, DEPTH=5, GRID=256, MAJORANT=8.0, MAJORANT_W=8.5, ALBEDO=0.9, G=0.3, FD_SPP=8,
         metric="Mpaths/s (density-grid medium, delta tracking, 1 spp per step)",
@@ -78,14 +78,14 @@ SCENES = {
                  "radiance cache (96-64x5-3 FP16 MLP, 12-band position encoding) answering primary hits, "
                  "1 training path per 32, 2^16 samples per frame in Adam steps of 2^14, lr 1e-2; "
                  "time budget = `steps` frames of the plain path tracer",
-        l2="inputs larger than L2 (scene 222 MB resident)"),
+        l2="inputs larger than L2 (scene 265 MB resident)"),
     "rmse": dict(
         W=1920, H=1080, DEPTH=8, GT_SPP=8192, PIXELS=16, SPP=(1, 4, 16, 64, 256),
         metric="Mpaths/s at equal RMSE vs an FP64 oracle (NEE path tracing, 1M-triangle scene)",
         workload="1M-triangle heightfield + 200 icospheres (2,024,000 tris), 1920x1080, depth 8; RMSE of 16 seeded "
                  "pixels against an 8192-spp FP64 oracle render of them (disjoint sample frames), at 1..256 spp, "
                  "for this library and for the reference's host build",
-        l2="inputs larger than L2 (scene 222 MB resident)"),
+        l2="inputs larger than L2 (scene 265 MB resident)"),
     "volume": dict(
         W=512, H=512, DEPTH=5,
         metric="Mpaths/s (RenderingMethod::VOLUME, 1 spp per step)",
@@ -370,11 +370,14 @@ def run_reference(args) -> int:
 # bench run (the bench never runs under ncu).  Each entry names the capture;
 # the per-kernel summary under profiles/ gives the full command.
 NCU_TRAFFIC = {
-    # k_extend, heightfield at 960x540 (the bench's scene, smaller frame):
-    # 68.5 B per ray on the depth-0 launch, scaled to the 7,769,878 rays of a
-    # 1920x1080 two-frame launch (traffic grows with the rays traced)
-    "k_extend heightfield": {"bytes_per_launch": 532.2e6,
-                             "capture": "ncu --set full -k regex:k_extend -s 8 -c 2, bench.py --resolution 960x540"},
+    # closest hits, heightfield at 960x540 (the bench's scene, smaller frame),
+    # four frames in one wavefront: 59.2 B per ray of the camera packets
+    # (k_extend_camera) and 83.3 B per ray of the first bounce (k_extend), scaled
+    # to the rays of a full wavefront's eight launches (16 frames of 2,073,600
+    # camera rays and 1,811,339 others)
+    "k_extend heightfield": {"bytes_per_launch": 547.3e6,
+                             "capture": "ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum -k regex:k_extend "
+                                        "-s 3 -c 3, render_frames(4) at 960x540, depth 2"},
     # k_rc_infer with component-major query records, one cached 4-frame
     # 960x540 wavefront (about 1.54 M queries): read 97.7 + write 9.3 B per
     # query (traffic per query does not depend on the frame size)
@@ -385,7 +388,7 @@ NCU_TRAFFIC = {
 
 
 def _read_traffic(scene):
-    """Recorded DRAM bytes per k_extend launch for `scene` (NCU_TRAFFIC), or None."""
+    """Recorded DRAM bytes per closest-hit launch for `scene` (NCU_TRAFFIC), or None."""
     rec = NCU_TRAFFIC.get(f"k_extend {scene}")
     return None if rec is None else rec["bytes_per_launch"]
 
@@ -553,19 +556,23 @@ def run_b200(args) -> int:
                                "primitive_tests": st["shadow_prims"] / max(1, st["shadow_rays"])}},
                 "stage_ms_per_step": {k: round(stages[k] / args.steps, 4)
                                       for k in ("camera", "extend", "shade", "connect", "accumulate")},
-                "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                             "frac": achieved / peak, "traffic": traffic, "peak_source": f"{peak_src} hbm_gbs",
-                             "kernel": "k_extend (closest hit), timed as the closest-hit stage of the one-stream pass, "
-                                       "which also holds the camera-ray packets and the per-path tail kernel",
+                "roofline": {"bound": "issue and cache latency (the reads are served by L1 and L2: achieved is the rate "
+                                      "at which the algorithm's reads are consumed, and may pass the DRAM peak)",
+                             "achieved": achieved, "peak": peak, "unit": "GB/s",
+                             "frac": achieved / peak, "traffic": traffic,
+                             "peak_source": f"{peak_src} hbm_gbs",
+                             "kernel": "closest-hit stage of the one-stream pass: k_extend_camera, k_extend and the "
+                                       "per-path tail kernel",
                              "bytes_per_launch": per_launch,
                              "bytes_model": "112*node_visits (7 float4 of a 4-wide node) + 48*triangle_tests + 96 per ray"},
-                "roofline_connect": {"bound": "hbm", "achieved": con_achieved, "peak": peak, "unit": "GB/s",
+                "roofline_connect": {"bound": "issue and cache latency", "achieved": con_achieved, "peak": peak, "unit": "GB/s",
                                      "frac": con_achieved / peak, "peak_source": f"{peak_src} hbm_gbs",
                                      "kernel": "k_connect (shadow rays, any hit), timed as the shadow-ray stage of the "
                                                "one-stream pass",
                                      "bytes_per_launch": con_per_launch,
                                      "bytes_model": "112*node_visits + 48*triangle_tests + 64 per shadow ray"},
-                "gpu_launches": stages["frames"] * (4 * DEPTH + 2),
+                # camera, per depth closest hit / shading / shadow rays, accumulation (no tail where frames overlap)
+                "gpu_launches": stages["frames"] * (3 * DEPTH + 2),
                 "device_errors": errors,
                 "scene": {"triangles": info["triangles"], "bvh_nodes": info["bvh_nodes"],
                           "device_mb": round(info["device_bytes"] / 2**20, 1)},
@@ -860,7 +867,8 @@ def run_medium(args) -> int:
                              "tracking": "weighted, q 0.5, majorant 8.5",
                              "outputs": f"{grid.size} voxel + {npar} parameter gradients",
                              "fd_check": fd},
-                "gpu_launches": stages["wavefronts"] * (4 * DEPTH + 2),
+                # camera, per depth closest hit / flight / two vertex kinds / transmittance / shadow rays, accumulation
+                "gpu_launches": stages["wavefronts"] * (6 * DEPTH + 2),
                 "device_errors": errors,
                 "clocks": clocks,
                 "reference_cuda": {"unavailable": "the reference has no density-grid medium (homogeneous only)"}}
@@ -1314,12 +1322,14 @@ def run_method(args) -> int:
                                  + 12 * args.steps),
                 "device_errors": r.error_count(), "clocks": clocks}
         if rec_ms is not None:
-            rec_bytes = 72.0 * W * H * 50 + 72.0 * W * H  # 50 passes of 5 reads + 1 write, init 6 reads + 3 writes
+            # per launch of 5 passes three images read and one written (borders aside); init 6 reads + 3 writes
+            rec_bytes = (48.0 * 10 + 108.0) * W * H
             line["roofline_reconstruction"] = {
                 "kernel": "k_gdpt_init + 10 x k_gdpt_opt (5 passes each)", "ms_per_step": rec_ms / args.steps,
                 "achieved": rec_bytes * args.steps / (rec_ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                 "frac": rec_bytes * args.steps / (rec_ms * 1e-3) / 1e9 / peak,
-                "note": "algorithmic 72 B per pixel and pass (50 passes); the kernel reads each image once per 5 passes, and the nine 3 MB images stay in L2"}
+                "note": "48 B per pixel and launch and 108 B for the initial pass; bound by issue and each block's latency, the "
+                        "nine 3 MB images stay in L2"}
         if world == 1 and not args.no_reference_cuda:
             try:
                 from oracle import bridge

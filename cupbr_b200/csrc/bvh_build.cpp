@@ -282,7 +282,7 @@ void build_bvh(const std::vector<PrimBox>* boxes, int ntypes, const uint32_t* sl
         }
         return n;
     };
-    // 4-wide nodes: breadth-first for the top levels (shared-memory staging),
+    // 4-wide nodes: breadth-first for the top levels,
     // depth-first below
     struct W4 { int32_t src; int32_t child[4]; int n; uint32_t depth; };
     std::vector<W4> order;

@@ -28,7 +28,7 @@ struct PrimBox {
 struct BvhBuildParams {
     int max_leaf = 4;         // primitives per leaf (<= BVH_MAX_LEAF)
     float trav_cost = 2.0f;   // SAH cost of one node step relative to one primitive test
-    int top_bfs_levels = 4;   // 4-wide levels laid out breadth-first at the front (shared-memory staging)
+    int top_bfs_levels = 4;   // 4-wide levels laid out breadth-first at the front
     bool device = true;       // build on the GPU (bvh_gpu.cu); false: build_bvh on the host (same arrays)
 };
 

@@ -16,8 +16,7 @@ namespace cupbr_b200 {
 // that reaches this is broken input (NaN densities, a zero majorant).
 constexpr int MEDIUM_MAX_EVENTS = 1 << 16;
 // Parameter gradients are accumulated per block in shared memory up to this
-// many entries (32 KB next to the 16 KB of staged BVH nodes), in global
-// memory beyond.
+// many entries (32 KB), in global memory beyond.
 constexpr uint32_t MEDIUM_SMEM_PARAMS = 8192;
 constexpr uint32_t MEDIUM_STATS = 5;
 

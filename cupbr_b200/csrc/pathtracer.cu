@@ -21,9 +21,8 @@
 // PathTracer.cu:37-41) stops early: its remaining contributions are all
 // zero and its RNG stream is private, so no other pixel changes.
 //
-// Queue slots are claimed with warp-aggregated atomics (one atomicAdd per
-// warp, ballot + popc for the lane offsets); the traversal kernels are
-// persistent (persistent_trace).
+// The shading stage claims queue slots once per block (BlockClaim); the
+// traversal kernels are persistent (persistent_trace).
 #include "pathtracer.hpp"
 
 #include "cache.hpp"
@@ -108,13 +107,15 @@ __global__ void __launch_bounds__(PT_TRACE_THREADS, 8) k_connect(DeviceScene S, 
                                   });
 }
 
-// 4 blocks of 256 per SM (64 registers; measured faster than the
-// unconstrained 92 registers at 2 blocks, despite a few spilled bytes).
-// Blocks of T rays sorted by material class.  Where the materials are of
-// several classes a large block fills more warps with one class (terrain 1080p x
-// 16 frames, T = 128 / 256 / 512: 47.7, 44.5, 42.7 ms); where there is one class
-// a small block waits less at its barriers (Cornell box, 16.8 M paths: 9.67,
-// 9.82, 10.28 ms).  shade_blocks chooses.
+// Blocks of T rays sorted by material class, 1024 threads per SM (64 registers,
+// a few bytes spilled; unconstrained registers leave half as many and are
+// slower).  Where the materials are of several classes a large block fills more
+// warps with one class (terrain 1080p x 16 frames, T = 128 / 256 / 512: 47.7, 44.5,
+// 42.7 ms; all materials 1280 x 720 x 16 4.28, 3.72, 3.46, with the physical
+// estimator and Russian roulette 3.92, 3.57, 3.42); where there is one class a
+// small block waits less at its barriers (Cornell box, 16.8 M paths: 9.67, 9.82,
+// 10.28 ms; with both options 1280 x 720 x 16 3.71, 3.78, 3.96).  Cached frames differ by
+// 2 % at most.  shade_blocks chooses.
 template <bool CACHE, bool PHYS, uint32_t T>
 __global__ void __launch_bounds__(T, 1024 / T) k_shade(DeviceScene S, PTFrame F, Workspace W, uint32_t depth, CacheFrame C) {
     shade_stage<CACHE, PHYS, true, false, T>(S, F, W, depth, C);

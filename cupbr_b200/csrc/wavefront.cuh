@@ -221,8 +221,7 @@ struct TraceShare {
 // Persistent traversal over a queue with per-lane dynamic fetch.  A warp's
 // lanes walk the tree in rounds of at most TRACE_NODE_STEPS node visits and
 // then one leaf: a bound on the visits, because a round that descends until
-// every lane holds a leaf runs as long as its slowest lane (9 of 32 lanes busy
-// on the 2M-triangle terrain's bounce rays; 13 with the bound).  Lanes whose
+// every lane holds a leaf runs as long as its slowest lane.  Lanes whose
 // ray is done wait until TRACE_REFILL of them (or the whole warp) can hand in
 // their results and take the next rays together; the warp claims the queue in
 // chunks, so a refill rarely waits for an atomic.  Entry i of the queue starts
