@@ -310,8 +310,16 @@ __device__ __forceinline__ void persistent_trace(const DeviceScene& S, const flo
     }
     if (overflow) atomicAdd(err_stack, 1u);
     if (COUNT) {
-        atomicAdd((unsigned long long*)&stats[0], (unsigned long long)tc.nodes);
-        atomicAdd((unsigned long long*)&stats[1], (unsigned long long)tc.tris);
+        // one addition per warp that has something to add: every warp of the grid
+        // comes by here, whatever the queue's length, and the additions to one
+        // counter complete one after the other (2 ms a frame of any size by lane)
+        unsigned long long nodes = tc.nodes, tris = tc.tris;
+        for (int o = 16; o > 0; o >>= 1) {
+            nodes += __shfl_down_sync(full, nodes, o);
+            tris += __shfl_down_sync(full, tris, o);
+        }
+        if (lane == 0 && nodes) atomicAdd((unsigned long long*)&stats[0], nodes);
+        if (lane == 0 && tris) atomicAdd((unsigned long long*)&stats[1], tris);
     }
 }
 
